@@ -31,6 +31,7 @@
 #include "fgmres.cuh"
 #include "kernels.cuh"
 #include "pcg_cluster.cuh"
+#include "pcg_resident.cuh"
 #include "persistent.cuh"
 #include "scalars.cuh"
 #include "step_vjp.cuh"
@@ -208,12 +209,17 @@ struct fugu_ctx {
   // instantiation with such a node fails, and those iterations run eagerly
   bool coop_graphs = true;
   bool capture_coop = false;  // the capture in progress holds a grid-wide launch
-  // cluster-resident PCG plan per precision (index 0 FP64, 1 FP32)
+  // PCG plans per precision (index 0 FP64, 1 FP32): one thread-block cluster,
+  // and the resident form over the whole device, which takes precedence in a
+  // context of its own (pcg())
   struct ClusterPlan {
     bool ok = false;
-    int C = 0, rows_per = 0, cpt = 0;
+    int C = 0, rows_per = 0, tpb = 0;
+    int form = 0;  // FP64: the resident kernel's shape; FP32: cells per strip (32: the lean kernel)
     size_t smem = 0;
   } pcgc[2];
+  PcgrPlan pcgg[2];
+  Exchange xch{};  // the grid form's exchange buffers (allocated with its plan)
   // CUDA graphs of the flexible-GMRES Arnoldi steps (graphs = 1), per
   // precision (0 FP64, 1 FP32) and step index j
   struct StepGraph {
@@ -417,26 +423,17 @@ void scalar_op(fugu_ctx* c, OpArgs op, bool check_active) {
   CKL("k_scalar_op");
 }
 
-// cluster-resident PCG: kernel for a cells-per-thread count
+// the kernel of a precision's cluster plan
 template <typename T>
-const void* pcgc_fn(int cpt) {
-  switch (cpt) {
-    case 1: return (const void*)k_pcg_cluster<T, 1>;
-    case 2: return (const void*)k_pcg_cluster<T, 2>;
-    case 4: return (const void*)k_pcg_cluster<T, 4>;
-    case 8: return (const void*)k_pcg_cluster<T, 8>;
-    case 16: return (const void*)k_pcg_cluster<T, 16>;
-    case 32:
-      if constexpr (sizeof(T) == 4) return (const void*)k_pcg_cluster<T, 32>;
-      break;
-  }
-  return nullptr;
+const void* pcgc_fn(int form) {
+  if constexpr (sizeof(T) == 8) return pcgr_fn<double, true>(form);
+  else return form == PCGC_LEAN_CPT ? (const void*)k_pcg_cluster_lean : pcg_column_fn(form);
 }
-template <typename T>
-cudaLaunchConfig_t pcgc_cfg(int C, size_t smem, cudaStream_t s, cudaLaunchAttribute* at) {
+// launch of C CTAs as one thread-block cluster
+cudaLaunchConfig_t cluster_cfg(int C, int tpb, size_t smem, cudaStream_t s, cudaLaunchAttribute* at) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C, 1, 1);
-  cfg.blockDim = dim3(PCGC_TPB, 1, 1);
+  cfg.blockDim = dim3(tpb, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -447,17 +444,44 @@ cudaLaunchConfig_t pcgc_cfg(int C, size_t smem, cudaStream_t s, cudaLaunchAttrib
   cfg.numAttrs = 1;
   return cfg;
 }
-template <typename T>
-cudaError_t launch_pcg_cluster(PcgClusterArgs<T> a, int C, int cpt, size_t smem, cudaStream_t s) {
-  cudaLaunchAttribute at[1];
-  cudaLaunchConfig_t cfg = pcgc_cfg<T>(C, smem, s, at);
-  void* args[] = {&a};
-  return cudaLaunchKernelExC(&cfg, pcgc_fn<T>(cpt), args);
+// the device's opt-in shared memory left for a kernel's dynamic part
+size_t smem_cap_of(const fugu_ctx* c, const void* fn) {
+  int optin = 0;
+  cudaFuncAttributes fa;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) != cudaSuccess ||
+      cudaFuncGetAttributes(&fa, fn) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return (size_t)optin - fa.sharedSizeBytes;
 }
-// Plan the cluster-resident PCG for precision T: up to 16 CTAs of PCGC_TPB
-// threads, every CTA's rows must fit the shared memory and the register
-// arrays (cpt <= 8 in FP64, <= 32 in FP32 with the lean variant above 16),
-// and the device must be able to co-schedule such a cluster.
+// Raise fn's dynamic shared-memory limit to smem_cap and check that the
+// device can co-schedule a cluster of C CTAs.  The limit is a property of the
+// kernel, shared by every context in the process, so it is always raised to
+// the device's maximum (never to one case's need, which would shrink it for
+// another).
+bool cluster_fits(fugu_ctx* c, const void* fn, int C, int tpb, size_t smem, size_t smem_cap) {
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap) != cudaSuccess ||
+      cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  cudaLaunchAttribute at[1];
+  cudaLaunchConfig_t cfg = cluster_cfg(C, tpb, smem, c->s, at);
+  int nclusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&nclusters, fn, &cfg) != cudaSuccess || nclusters < 1) {
+    cudaGetLastError();
+    return false;
+  }
+  return true;
+}
+// Plan one case's cluster PCG: up to max_cluster CTAs, every CTA's rows in
+// registers and shared memory, and the device able to co-schedule the
+// cluster.  FP64 (resident kernel): fewer CTAs when the grid gives each fewer
+// than 128 segments, since the exchange and the idle lanes then cost more than
+// the shorter serial part gains; its sums do not depend on the partition.
+// FP32 (column strips): as many CTAs as max_cluster allows and the shortest
+// strips, which fix the order of its sums.
 template <typename T>
 void plan_pcg_cluster(fugu_ctx* c, fugu_ctx::ClusterPlan& pl) {
   pl = fugu_ctx::ClusterPlan{};
@@ -465,45 +489,58 @@ void plan_pcg_cluster(fugu_ctx* c, fugu_ctx::ClusterPlan& pl) {
   if (env && std::strcmp(env, "grid") == 0) return;
   const int nx = c->prm.nx, ny = c->prm.ny;
   const int cmax = ny < c->max_cluster ? ny : c->max_cluster;
-  const int rows_per = (ny + cmax - 1) / cmax;
-  const int C = (ny + rows_per - 1) / rows_per;
-  // every thread owns one column and a strip of cpt rows: nx * strips <= TPB
-  if (nx > PCGC_TPB) return;
-  int cpt = 1;
-  while ((long)nx * ((rows_per + cpt - 1) / cpt) > PCGC_TPB) cpt *= 2;
-  const int cpt_max = sizeof(T) == 8 ? 8 : 32;
-  if (cpt > cpt_max) return;
-  const void* fn = pcgc_fn<T>(cpt);
-  // The dynamic shared-memory limit is a property of the kernel, shared by
-  // every context in the process, so it is always raised to the device's
-  // maximum (never to one case's need, which would shrink it for another).
-  int optin = 0;
-  cudaFuncAttributes fa;
-  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) != cudaSuccess ||
-      cudaFuncGetAttributes(&fa, fn) != cudaSuccess) {
-    cudaGetLastError();
-    return;
+  if constexpr (sizeof(T) == 8) {
+    const long segs = (long)ny * ((nx + 1) / 2);
+    const PcgrPlan p = pcgr_plan<double>(nx, ny, (int)std::min<long>(cmax, std::max<long>(2, segs / 128)));
+    if (!p.ok) return;
+    pl.C = p.G;
+    pl.rows_per = p.rows_per;
+    pl.tpb = p.tpb;
+    pl.form = p.shape;
+    pl.smem = p.smem;
+  } else {
+    // every thread owns one column and a strip of cpt rows
+    if (nx > PCGC_TPB) return;
+    pl.rows_per = (ny + cmax - 1) / cmax;
+    pl.C = (ny + pl.rows_per - 1) / pl.rows_per;
+    int cpt = 1;
+    while ((long)nx * ((pl.rows_per + cpt - 1) / cpt) > PCGC_TPB) cpt *= 2;
+    if (cpt > PCGC_LEAN_CPT) return;
+    pl.form = cpt;
+    pl.tpb = cpt == PCGC_LEAN_CPT ? PCGC_TPB : pcg_column_tpb(nx, pl.rows_per, cpt);
+    pl.smem = sizeof(float) * (size_t)(cpt == PCGC_LEAN_CPT ? pcgc_smem_elems(nx, pl.rows_per)
+                                                            : pcgcol_smem_elems(nx, pl.rows_per, cpt));
   }
-  const size_t smem = sizeof(T) * (size_t)pcgc_smem_elems<T>(nx, rows_per, cpt);
-  const size_t smem_cap = (size_t)optin - fa.sharedSizeBytes;
-  if (smem > smem_cap) return;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap) != cudaSuccess ||
-      cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-    cudaGetLastError();
-    return;
-  }
-  cudaLaunchAttribute at[1];
-  cudaLaunchConfig_t cfg = pcgc_cfg<T>(C, smem, c->s, at);
-  int nclusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&nclusters, fn, &cfg) != cudaSuccess || nclusters < 1) {
-    cudaGetLastError();
-    return;
-  }
-  pl.ok = true;
-  pl.C = C;
-  pl.rows_per = rows_per;
-  pl.cpt = cpt;
-  pl.smem = smem;
+  const void* fn = pcgc_fn<T>(pl.form);
+  const size_t cap = smem_cap_of(c, fn);
+  pl.ok = pl.smem <= cap && cluster_fits(c, fn, pl.C, pl.tpb, pl.smem, cap);
+}
+// Plan the resident PCG over the whole device for a context of its own (one
+// cooperative launch; a batch's cases share the device, so they keep the
+// cluster form).  About 1,024 cells per CTA, up to one CTA per SM: more CTAs
+// shorten the serial part, fewer shorten the exchange.  FP32: where no
+// cluster holds the grid.  FP64: also in place of the cluster above 32,768
+// cells; measured on a B200 (us per iteration, cluster / grid): 203 x 125
+// 4.06 / 4.20, 128 x 256 4.10 / 4.00, 256 x 256 5.99 / 4.55.
+constexpr long PCGR_GRID_CELLS = 32768;
+template <typename T>
+void plan_pcg_grid(fugu_ctx* c, PcgrPlan& p) {
+  p = PcgrPlan{};
+  const long cells = (long)c->prm.nx * c->prm.ny;
+  const char* env = std::getenv("FUGU_PCG");  // "grid" and "cluster" name the other kernels
+  if (env && (std::strcmp(env, "grid") == 0 || std::strcmp(env, "cluster") == 0)) return;
+  if (c->coop_as_cluster) return;
+  if (c->pcgc[sizeof(T) == 8 ? 0 : 1].ok && (sizeof(T) == 4 || cells <= PCGR_GRID_CELLS)) return;
+  const long most = std::min<long>(std::min(c->nsm, c->max_coop), c->prm.ny);
+  p = pcgr_plan<T>(c->prm.nx, c->prm.ny, (int)std::min<long>(most, std::max<long>(1, cells / 1024)));
+  if (!p.ok) return;
+  const void* fn = pcgr_fn<T, false>(p.shape);
+  const size_t cap = smem_cap_of(c, fn);
+  int occ = 0;
+  p.ok = p.smem <= cap &&
+         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) == cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, p.tpb, p.smem) == cudaSuccess && occ >= 1;
+  if (!p.ok) cudaGetLastError();
 }
 
 // Launch a persistent kernel whose CTAs wait on one another at grid
@@ -514,11 +551,11 @@ void plan_pcg_cluster(fugu_ctx* c, fugu_ctx::ClusterPlan& pl) {
 // as one thread-block cluster (at most 8 CTAs), whose CTAs the hardware
 // schedules together or not at all.  Both forms are launch attributes, so a
 // stream capture records them as attributes of the kernel node.
-void launch_coop(fugu_ctx* c, const void* fn, int grid, void** args) {
+void launch_coop(fugu_ctx* c, const void* fn, int grid, void** args, int tpb = PCG_TPB, size_t smem = 0) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(PCG_TPB);
-  cfg.dynamicSmemBytes = 0;
+  cfg.blockDim = dim3(tpb);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = c->s;
   cudaLaunchAttribute at[1];
   if (c->coop_as_cluster) {
@@ -596,13 +633,35 @@ void pcg(fugu_ctx* c, PcgWork<T>& w, T* phi, const T* rhs, double tol, int max_i
     a.extra_arrivals = 1;
     c->test_spin_limit = 0;
   }
-  if (cp.ok && !armed) {
-    PcgClusterArgs<T> ca;
-    ca.g = c->g;
-    ca.rhs = rhs; ca.cx = w.cx; ca.cy = w.cy; ca.dinv = w.dinv; ca.phi = phi;
-    ca.out = c->pcg_out; ca.active = active; ca.tol = tol; ca.max_iter = max_iter;
-    ca.phi_zero = phi_zero ? 1 : 0; ca.rows_per = cp.rows_per; ca.timed = a.timed;
-    CK(launch_pcg_cluster<T>(ca, cp.C, cp.cpt, cp.smem, c->s));
+  const PcgrPlan& gp = c->pcgg[sizeof(T) == 8 ? 0 : 1];
+  if (gp.ok || (cp.ok && !armed)) {
+    PcgResArgs<T> ra{};
+    ra.g = c->g;
+    ra.rhs = rhs; ra.cx = w.cx; ra.cy = w.cy; ra.dinv = w.dinv; ra.phi = phi;
+    ra.out = c->pcg_out; ra.active = active; ra.tol = tol; ra.max_iter = max_iter;
+    ra.phi_zero = phi_zero ? 1 : 0; ra.timed = a.timed;
+    ra.rows_per = gp.ok ? gp.rows_per : cp.rows_per;
+    if (gp.ok) {
+      ra.x = c->xch;
+      ra.err = &c->gs->error;
+      ra.spin_limit = a.spin_limit;
+      ra.extra_arrivals = a.extra_arrivals;
+      void* args[] = {&ra};
+      launch_coop(c, pcgr_fn<T, false>(gp.shape), gp.G, args, gp.tpb, gp.smem);
+    } else {
+      PcgClusterArgs ca{};
+      void* args[] = {&ra};
+      if constexpr (sizeof(T) == 4) {
+        ca.g = ra.g;
+        ca.rhs = ra.rhs; ca.cx = ra.cx; ca.cy = ra.cy; ca.dinv = ra.dinv; ca.phi = ra.phi;
+        ca.out = ra.out; ca.active = ra.active; ca.tol = ra.tol; ca.max_iter = ra.max_iter;
+        ca.phi_zero = ra.phi_zero; ca.rows_per = ra.rows_per; ca.timed = ra.timed;
+        args[0] = &ca;
+      }
+      cudaLaunchAttribute at[1];
+      cudaLaunchConfig_t cfg = cluster_cfg(cp.C, cp.tpb, cp.smem, c->s, at);
+      CK(cudaLaunchKernelExC(&cfg, pcgc_fn<T>(cp.form), args));
+    }
   } else {
     CK(cudaMemsetAsync(c->gs, 0, sizeof(GridSync), c->s));
     void* args[] = {&a};
@@ -811,7 +870,9 @@ struct KrylovResult {
 void graph_prof_read(fugu_ctx* c);
 
 // Krylov iterations of precision pi (0 FP64, 1 FP32) replay from graphs
-bool graphs_on(const fugu_ctx* c, int pi) { return c->prm.graphs == 1 && (c->pcgc[pi].ok || c->coop_graphs); }
+bool graphs_on(const fugu_ctx* c, int pi) {
+  return c->prm.graphs == 1 && ((c->pcgc[pi].ok && !c->pcgg[pi].ok) || c->coop_graphs);
+}
 
 // Run body() on the context's stream from a CUDA graph: the captured graph
 // is replayed while key (every value its launches depend on) is unchanged;
@@ -1668,6 +1729,18 @@ void create(fugu_ctx* c) {
   if (c->pcg_grid < 1 || c->svof_grid < 1) throw ApiError{FUGU_ECUDA, "no co-resident grid for persistent kernels"};
   plan_pcg_cluster<double>(c, c->pcgc[0]);
   plan_pcg_cluster<float>(c, c->pcgc[1]);
+  plan_pcg_grid<double>(c, c->pcgg[0]);
+  plan_pcg_grid<float>(c, c->pcgg[1]);
+  if (c->pcgg[0].ok || c->pcgg[1].ok) {
+    // one slot per CTA and one that is never written (failure-detection test);
+    // a halo row takes a word per float, two per double
+    Exchange& x = c->xch;
+    x.nslots = std::max(c->pcgg[0].ok ? c->pcgg[0].G : 0, c->pcgg[1].ok ? c->pcgg[1].G : 0) + 1;
+    x.halo_words = (long)((c->prm.nx + 1) / 2 + 1) * 4;
+    x.epoch = dalloc<unsigned int>(c, 1);
+    x.sum = dalloc<ulonglong2>(c, 2L * x.nslots * GX_NV);
+    x.halo = dalloc<unsigned long long>(c, 4L * x.nslots * x.halo_words);
+  }
   // the multi-sweep Jacobi tiles of FP64 need more than the default 48 KB
   CK(cudaFuncSetAttribute((const void*)k_jacobi_multi<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)sizeof(JmSmem<double>)));
@@ -2830,8 +2903,12 @@ double time_pcg_iter(fugu_ctx* c, PcgWork<T>& w, T* phi, const T* rhs, int iters
 // Autotune the PCG cluster size of context c for precision T: candidates
 // 2, 4, 8, 16 CTAs (those the planner accepts).  The Poisson coefficients
 // are those of uniform unit density, the right-hand side a smooth mode; the
-// iteration cost does not depend on the values.  Returns the chosen size
-// (0 when no cluster plan fits: the grid-wide kernel is used).
+// iteration cost does not depend on the values.  In FP32, strips of more
+// than PCGC_COL_REG cells are candidates only when no size gives shorter
+// ones: a batch runs about one case per host thread, so its cases rarely fill
+// the device and a case's latency counts (128 x 256: 8 CTAs 2.4 us per
+// iteration, 4 CTAs 4.0).  Returns the chosen size (0 when no cluster plan
+// fits: the grid-wide kernel is used).
 template <typename T>
 int tune_cluster(fugu_ctx* c) {
   const int idx = sizeof(T) == 8 ? 0 : 1;
@@ -2852,10 +2929,19 @@ int tune_cluster(fugu_ctx* c) {
   sync(c);  // the host vectors go out of scope
   int best = 0;
   double best_cost = 0.0;
+  bool has_short = false;
+  if constexpr (sizeof(T) == 4) {
+    for (int C = 2; C <= 16; C *= 2) {
+      c->max_cluster = C;
+      plan_pcg_cluster<T>(c, c->pcgc[idx]);
+      has_short = has_short || (c->pcgc[idx].ok && c->pcgc[idx].C == C && c->pcgc[idx].form <= PCGC_COL_REG);
+    }
+  }
   for (int C = 2; C <= 16; C *= 2) {
     c->max_cluster = C;
     plan_pcg_cluster<T>(c, c->pcgc[idx]);
     if (!c->pcgc[idx].ok || c->pcgc[idx].C != C) continue;
+    if (has_short && c->pcgc[idx].form > PCGC_COL_REG) continue;
     const double cost = C * time_pcg_iter<T>(c, w, phi, rhs, 64);
     if (!best || cost < best_cost) {
       best = C;
@@ -2943,7 +3029,7 @@ int lockstep_create(fugu_batch* b, int group_max) {
       return FUGU_EINVAL;
     }
     const fugu_ctx::ClusterPlan& pl = c->pcgc[pi];
-    const std::array<long, 4> key = {pl.C, pl.cpt, pl.rows_per, (long)pl.smem};
+    const std::array<long, 4> key = {pl.C, pl.form, pl.rows_per, (long)pl.smem};
     auto it = by_class.find(key);
     if (it == by_class.end()) {
       class_order.push_back(key);

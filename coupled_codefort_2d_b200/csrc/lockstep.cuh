@@ -28,6 +28,7 @@
 #include "fgmres.cuh"
 #include "kernels.cuh"
 #include "pcg_cluster.cuh"
+#include "pcg_resident.cuh"
 #include "scalars.cuh"
 
 namespace fugu {
@@ -685,16 +686,18 @@ __global__ void __launch_bounds__(MT_TPB) k_ls_matvec(const LsCase<T>* cs, const
 }
 
 // cluster-resident PCG of the PCD on V_j's pressure block for the cases of
-// one grid class: cluster q solves case cls[q] (k_pcg_cluster)
-template <typename T, int CPT>
-__global__ void __launch_bounds__(PCGC_TPB, 1) k_ls_pcg(const LsCase<T>* cs, const LsDyn* dyn, const int* cls,
-                                                       int rows_per, int j) {
-  const int C = (int)cgc::this_cluster().num_blocks();
+// one grid class: cluster q solves case cls[q].  FORM is the plan's: FP64 the
+// shape of k_pcg_resident, FP32 the strip of k_pcg_column (32: the lean kernel).
+template <typename T, int FORM>
+__global__ void __launch_bounds__(sizeof(T) == 8 ? pcgr_shape(FORM).tpb : PCGC_TPB, 1)
+    k_ls_pcg(const LsCase<T>* cs, const LsDyn* dyn, const int* cls, int rows_per, int j) {
+  cgc::cluster_group cl = cgc::this_cluster();
+  const int C = (int)cl.num_blocks();
   const int s = cls[blockIdx.x / C];
   const LsCase<T>& c = cs[s];
   const LsDyn& d = dyn[s];
   if (!d.run || !c.ks->active) return;  // the same for every CTA of the cluster
-  PcgClusterArgs<T> a;
+  std::conditional_t<sizeof(T) == 8, PcgResArgs<double>, PcgClusterArgs> a{};
   a.g = c.g;
   a.rhs = c.V + (long)j * 3 * c.n + 2 * c.n;
   a.cx = c.cx;
@@ -708,8 +711,36 @@ __global__ void __launch_bounds__(PCGC_TPB, 1) k_ls_pcg(const LsCase<T>* cs, con
   a.phi_zero = 1;
   a.rows_per = rows_per;
   a.timed = 0;
-  if constexpr (pcgc_one_reduction<T>(CPT)) pcg_cluster_body_1r<CPT>(a);
-  else pcg_cluster_body<T, CPT>(a);
+  if constexpr (sizeof(T) == 8) {
+    constexpr PcgrShape sh = pcgr_shape(FORM);
+    pcgr_body<T, sh.seg, sh.tpb, true>(a, (int)cl.block_rank(), C);
+  } else if constexpr (FORM == PCGC_LEAN_CPT) {
+    pcg_cluster_lean_body(a);
+  } else {
+    pcg_column_body<FORM>(a, (int)cl.block_rank(), C);
+  }
+}
+template <typename T>
+const void* ls_pcg_fn(int form) {
+  if constexpr (sizeof(T) == 8) {
+    switch (form) {
+      case 0: return (const void*)k_ls_pcg<T, 0>;
+      case 1: return (const void*)k_ls_pcg<T, 1>;
+      case 2: return (const void*)k_ls_pcg<T, 2>;
+      case 3: return (const void*)k_ls_pcg<T, 3>;
+      case 4: return (const void*)k_ls_pcg<T, 4>;
+    }
+  } else {
+    switch (form) {
+      case 1: return (const void*)k_ls_pcg<T, 1>;
+      case 2: return (const void*)k_ls_pcg<T, 2>;
+      case 4: return (const void*)k_ls_pcg<T, 4>;
+      case 8: return (const void*)k_ls_pcg<T, 8>;
+      case 16: return (const void*)k_ls_pcg<T, 16>;
+      case 32: return (const void*)k_ls_pcg<T, 32>;
+    }
+  }
+  return nullptr;
 }
 
 }  // namespace fugu

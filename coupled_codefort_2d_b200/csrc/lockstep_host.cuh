@@ -34,7 +34,8 @@ namespace {
   } while (0)
 
 struct LsClass {
-  int C = 0, cpt = 0, rows_per = 0;
+  int C = 0, rows_per = 0, tpb = 0;
+  const void* fn = nullptr;  // the class's PCG kernel
   size_t smem = 0;
   std::vector<int> cases;
   int* d_list = nullptr;
@@ -221,12 +222,13 @@ struct Lockstep : LockstepBase {
       r.visc = c->prm.pcd_visc_scale;
       // PCG grid class: the cluster plan of the case's inner precision
       const fugu_ctx::ClusterPlan& pl = c->pcgc[pi];
-      const std::array<long, 4> key = {pl.C, pl.cpt, pl.rows_per, (long)pl.smem};
+      const std::array<long, 4> key = {pl.C, pl.form, pl.rows_per, (long)pl.smem};
       auto it = cls_of.find(key);
       if (it == cls_of.end()) {
         LsClass k;
         k.C = pl.C;
-        k.cpt = pl.cpt;
+        k.fn = ls_pcg_fn<T>(pl.form);
+        k.tpb = pl.tpb;
         k.rows_per = pl.rows_per;
         k.smem = pl.smem;
         classes.push_back(k);
@@ -260,7 +262,7 @@ struct Lockstep : LockstepBase {
     for (auto& k : classes) {
       CK(cudaMalloc(&k.d_list, sizeof(int) * k.cases.size()));
       CK(cudaMemcpy(k.d_list, k.cases.data(), sizeof(int) * k.cases.size(), cudaMemcpyHostToDevice));
-      const void* fn = pcg_fn(k.cpt);
+      const void* fn = k.fn;
       int optin = 0;
       CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
       cudaFuncAttributes fa;
@@ -281,20 +283,6 @@ struct Lockstep : LockstepBase {
     }
     graphs.resize(m);
     warm_grids();
-  }
-
-  const void* pcg_fn(int cpt) {
-    switch (cpt) {
-      case 1: return (const void*)k_ls_pcg<T, 1>;
-      case 2: return (const void*)k_ls_pcg<T, 2>;
-      case 4: return (const void*)k_ls_pcg<T, 4>;
-      case 8: return (const void*)k_ls_pcg<T, 8>;
-      case 16: return (const void*)k_ls_pcg<T, 16>;
-      case 32:
-        if constexpr (sizeof(T) == 4) return (const void*)k_ls_pcg<T, 32>;
-        break;
-    }
-    throw ApiError{FUGU_EINVAL, "lockstep batch: no PCG kernel for this cluster plan"};
   }
 
   // co-resident CTAs of a family kernel (its persistent grid)
@@ -382,7 +370,7 @@ struct Lockstep : LockstepBase {
       if (k > 0) CK(cudaStreamWaitEvent(st, ev_fork, 0));
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)(cl.C * cl.cases.size()), 1, 1);
-      cfg.blockDim = dim3(PCGC_TPB, 1, 1);
+      cfg.blockDim = dim3(cl.tpb, 1, 1);
       cfg.dynamicSmemBytes = cl.smem;
       cfg.stream = st;
       cudaLaunchAttribute at[1];
@@ -397,7 +385,7 @@ struct Lockstep : LockstepBase {
       const int* a2 = cl.d_list;
       int a3 = cl.rows_per, a4 = j;
       void* args[] = {&a0, &a1, &a2, &a3, &a4};
-      CK(cudaLaunchKernelExC(&cfg, pcg_fn(cl.cpt), args));
+      CK(cudaLaunchKernelExC(&cfg, cl.fn, args));
       ++launches;
       if (k > 0) {
         CK(cudaEventRecord(ev_join[k], st));
