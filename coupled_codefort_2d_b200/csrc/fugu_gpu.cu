@@ -363,7 +363,7 @@ void matvec(fugu_ctx* c, const CoefBufs<T>& cb, const SolveOpt& o, Trip<T> X, Tr
   if (c->adj_on) {  // adjoint solve: the sign-conjugated transpose from the probed stencil
     if constexpr (std::is_same<T, double>::value) {
       Box b = box_launch(c->g);
-      k_adj_apply_t<<<b.grid, b.block, 0, c->s>>>(c->g, c->n, c->adj_val, X.base, Y.base, -1.0, active,
+      k_adj_apply_t<<<dim3(b.grid.x, b.grid.y, 3), b.block, 0, c->s>>>(c->g, c->n, c->adj_val, X.base, Y.base, -1.0, active,
                                                    &c->ks->matvecs);
       CKL("k_adj_apply_t");
       return;
@@ -2181,7 +2181,7 @@ void adj_assemble(fugu_ctx* c, const CoefBufs<double>& cb, const SolveOpt& o, do
         CKL("k_adj_probe_set");
         vbcs(c, X.u, X.v, 0.0);
         matvec<double>(c, cb, o, X, Y, dt, nullptr);
-        k_adj_probe_collect<<<b.grid, b.block, 0, c->s>>>(c->g, Y.base, c->n, cc, qx, qy, a, bb, c->adj_val,
+        k_adj_probe_collect<<<dim3(b.grid.x, b.grid.y, 3), b.block, 0, c->s>>>(c->g, Y.base, c->n, cc, qx, qy, a, bb, c->adj_val,
                                                           c->adj_err);
         CKL("k_adj_probe_collect");
       }
@@ -2236,6 +2236,7 @@ KrylovResult adjoint_solve_dev(fugu_ctx* c, const CoefBufs<double>& cb, const So
 // solve's stage reads C_smooth three cells away (curvature then CSF) and the
 // coefficients two; the wall BCs mirror up to four cells (u(-2) = -u(2)).
 constexpr int VJP_RA = 2, VJP_RB = 4, VJP_RG = 4;
+static_assert(VJP_RG == VJP_RB, "k_vjp_gather is built for two reaches");
 
 void vjp_alloc(fugu_ctx* c) {
   VjpWork& w = c->vjp;
@@ -2266,8 +2267,10 @@ void vjp_pack(fugu_ctx* c, const double* x, ad::Dual* out, int mask, bool seeded
 void vjp_gather(fugu_ctx* c, const VjpOut& o, int mask, int s, int a, int b, int R, double* xbar) {
   const int ti = (c->g.P - a + s - 1) / s, tj = (c->g.R - b + s - 1) / s;
   if (ti <= 0 || tj <= 0) return;
-  const dim3 blk(32, 4), grd((ti + 31) / 32, (tj + 3) / 4);
-  k_vjp_gather<<<grd, blk, 0, c->s>>>(c->g, o, mask, s, a, b, R, xbar);
+  const int nb = (ti * tj + VJPG_WARPS - 1) / VJPG_WARPS;
+  if (R == VJP_RA) k_vjp_gather<VJP_RA><<<nb, 32 * VJPG_WARPS, 0, c->s>>>(c->g, o, mask, s, a, b, ti, tj, xbar);
+  else if (R == VJP_RB) k_vjp_gather<VJP_RB><<<nb, 32 * VJPG_WARPS, 0, c->s>>>(c->g, o, mask, s, a, b, ti, tj, xbar);
+  else throw ApiError{FUGU_EINVAL, "vjp_gather: no kernel for this reach"};
   CKL("k_vjp_gather");
 }
 
@@ -2681,7 +2684,8 @@ int fugu_matvec_coupled_t(fugu_ctx* c, const double* Y_u, const double* Y_v, con
     Trip<double> Y = ST(c, 0), X = ST(c, 1);
     up_trip(c, Y, Y_u, Y_v, Y_p);
     Box b = box_launch(c->g);
-    k_adj_apply_t<<<b.grid, b.block, 0, c->s>>>(c->g, c->n, c->adj_val, Y.base, X.base, 1.0, nullptr, nullptr);
+    k_adj_apply_t<<<dim3(b.grid.x, b.grid.y, 3), b.block, 0, c->s>>>(c->g, c->n, c->adj_val, Y.base, X.base, 1.0,
+                                                                     nullptr, nullptr);
     CKL("k_adj_apply_t");
     down_trip(c, X, X_u, X_v, X_p);
     sync(c);
