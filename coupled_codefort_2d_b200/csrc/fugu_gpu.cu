@@ -35,6 +35,7 @@
 #include "persistent.cuh"
 #include "scalars.cuh"
 #include "step_vjp.cuh"
+#include "svof_cluster.cuh"
 
 using namespace fugu;
 
@@ -219,6 +220,12 @@ struct fugu_ctx {
     size_t smem = 0;
   } pcgc[2];
   PcgrPlan pcgg[2];
+  // SVOF filter in one cluster (svof_cluster.cuh); not ok: k_svof
+  struct SvofPlan {
+    bool ok = false;
+    int C = 0, rows_per = 0, cpt = 0;
+    size_t smem = 0;
+  } svofc;
   Exchange xch{};  // the grid form's exchange buffers (allocated with its plan)
   // CUDA graphs of the flexible-GMRES Arnoldi steps (graphs = 1), per
   // precision (0 FP64, 1 FP32) and step index j
@@ -541,6 +548,29 @@ void plan_pcg_grid(fugu_ctx* c, PcgrPlan& p) {
          cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) == cudaSuccess &&
          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, p.tpb, p.smem) == cudaSuccess && occ >= 1;
   if (!p.ok) cudaGetLastError();
+}
+
+// Plan the SVOF filter's cluster: about 512 cells per CTA, up to max_cluster
+// CTAs, each (the last one too) with at least the SVOF_T rows its neighbours keep
+void plan_svof(fugu_ctx* c, fugu_ctx::SvofPlan& pl) {
+  pl = fugu_ctx::SvofPlan{};
+  const int nx = c->prm.nx, ny = c->prm.ny;
+  if (nx > SVOFC_TPB) return;
+  const long want = std::min<long>(std::min(c->max_cluster, ny / SVOF_T), std::max(1L, (long)nx * ny / 512));
+  for (int C = (int)want; C >= 1; --C) {
+    const int rows_per = (ny + C - 1) / C, n = (ny + rows_per - 1) / rows_per, last = ny - (n - 1) * rows_per;
+    if (last < SVOF_T) continue;
+    pl.C = n;
+    pl.rows_per = rows_per;
+    break;
+  }
+  if (pl.C < 1) return;
+  pl.cpt = svofc_cpt(nx, pl.rows_per);
+  if (!pl.cpt) return;
+  const void* fn = svof_cluster_fn(pl.cpt);
+  pl.smem = sizeof(double) * (size_t)svofc_smem_elems(nx, pl.cpt);
+  const size_t cap = smem_cap_of(c, fn);
+  pl.ok = pl.smem <= cap && cluster_fits(c, fn, pl.C, SVOFC_TPB, pl.smem, cap);
 }
 
 // Launch a persistent kernel whose CTAs wait on one another at grid
@@ -1433,6 +1463,21 @@ void vof(fugu_ctx* c, const double* cin, double* cout, const double* u, const do
   halo(c, cout, K_CELL);
 }
 
+// the filter's kernel on the context's stream
+void svof_launch(fugu_ctx* c, SvofArgs& a) {
+  if (c->svofc.ok) {
+    SvofClusterArgs ca{a, c->svofc.rows_per};
+    void* args[] = {&ca};
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg = cluster_cfg(c->svofc.C, SVOFC_TPB, c->svofc.smem, c->s, at);
+    CK(cudaLaunchKernelExC(&cfg, svof_cluster_fn(c->svofc.cpt), args));
+  } else {
+    CK(cudaMemsetAsync(c->gs, 0, sizeof(GridSync), c->s));
+    void* args[] = {&a};
+    launch_coop(c, (const void*)k_svof, c->svof_grid, args);
+  }
+  ++c->launches;
+}
 // svof_helmholtz_filter (mod_vof.f90:145-194); returns nothing, adds the
 // iteration count to c->svof_iters
 void svof(fugu_ctx* c, const double* craw, double* cs, double* work, double delta, int max_iter, double tol) {
@@ -1450,10 +1495,7 @@ void svof(fugu_ctx* c, const double* craw, double* cs, double* work, double delt
   a.gs = c->gs;
   a.iters = c->svof_iters;
   a.status = c->svof_status;
-  CK(cudaMemsetAsync(c->gs, 0, sizeof(GridSync), c->s));
-  void* args[] = {&a};
-  launch_coop(c, (const void*)k_svof, c->svof_grid, args);
-  ++c->launches;
+  svof_launch(c, a);
 }
 
 void curvature(fugu_ctx* c, const double* cs, double* kc) {
@@ -1729,6 +1771,7 @@ void create(fugu_ctx* c) {
   if (c->pcg_grid < 1 || c->svof_grid < 1) throw ApiError{FUGU_ECUDA, "no co-resident grid for persistent kernels"};
   plan_pcg_cluster<double>(c, c->pcgc[0]);
   plan_pcg_cluster<float>(c, c->pcgc[1]);
+  plan_svof(c, c->svofc);
   plan_pcg_grid<double>(c, c->pcgg[0]);
   plan_pcg_grid<float>(c, c->pcgg[1]);
   if (c->pcgg[0].ok || c->pcgg[1].ok) {
@@ -2477,10 +2520,7 @@ void step_vjp(fugu_ctx* c, double dt, int step_idx, const fugu_step_opts* o, con
     a.gs = c->gs;
     a.iters = w.svof_it;
     a.status = c->svof_status;
-    CK(cudaMemsetAsync(c->gs, 0, sizeof(GridSync), c->s));
-    void* args[] = {&a};
-    launch_coop(c, (const void*)k_svof, c->svof_grid, args);
-    ++c->launches;
+    svof_launch(c, a);
     Box bx = box_launch(g);
     k_add_interior<<<bx.grid, bx.block, 0, c->s>>>(g, w.t1, w.b_c1);
     CKL("k_add_interior");
