@@ -14,7 +14,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libfugu_gpu.so")
 SOURCES = ["fugu_gpu.cu"]
-HEADERS = ["fugu_internal.cuh", "kernels.cuh", "persistent.cuh", "pcg_cluster.cuh", "pcg_resident.cuh", "pcg_exchange.cuh", "svof_cluster.cuh", "scalars.cuh", "fgmres.cuh", "adjoint.cuh",
+HEADERS = ["fugu_internal.cuh", "kernels.cuh", "persistent.cuh", "pcg_cluster.cuh", "pcg_resident.cuh", "pcg_exchange.cuh", "smooth_tile.cuh", "svof_cluster.cuh", "scalars.cuh", "fgmres.cuh", "adjoint.cuh",
            "dual.cuh", "step_vjp.cuh", "lockstep.cuh", "lockstep_host.cuh"]
 
 NVCC_FLAGS = [

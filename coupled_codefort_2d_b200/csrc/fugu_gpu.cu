@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <array>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -34,6 +35,7 @@
 #include "pcg_resident.cuh"
 #include "persistent.cuh"
 #include "scalars.cuh"
+#include "smooth_tile.cuh"
 #include "step_vjp.cuh"
 #include "svof_cluster.cuh"
 
@@ -626,7 +628,8 @@ void prof_drain(fugu_ctx* c) {
   c->ev_pcg.clear();
 }
 
-// persistent PCG (solve_poisson_pressure)
+// persistent PCG (solve_poisson_pressure).  phi_zero: phi counts as zero on
+// entry; its cells need not be, its ghosts are (no PCG writes those then)
 template <typename T>
 void pcg(fugu_ctx* c, PcgWork<T>& w, T* phi, const T* rhs, double tol, int max_iter, bool phi_zero,
          const int* active) {
@@ -694,6 +697,7 @@ void pcg(fugu_ctx* c, PcgWork<T>& w, T* phi, const T* rhs, double tol, int max_i
     }
   } else {
     CK(cudaMemsetAsync(c->gs, 0, sizeof(GridSync), c->s));
+    if (phi_zero) CK(cudaMemsetAsync(phi, 0, sizeof(T) * c->n, c->s));  // updated in place
     void* args[] = {&a};
     if constexpr (sizeof(T) == 4) {
       // the FP32 inner solve: one grid barrier per iteration
@@ -728,11 +732,8 @@ void poisson_coefs(fugu_ctx* c, PcgWork<T>& w, const double* rho_u, const double
 // one-thread-per-element kernels.  The size rule, from CUDA-event timings on
 // a B200 (FP32, us per launch): the PCD steps and single sweeps gain from
 // 1024^2 up (k_pcd_zwork 8.2 -> 6.2, one Jacobi sweep 12.3 -> 10.2) and lose
-// below (a sweep at 512^2 4.7 -> 5.7); against the staged multi-sweep kernel
-// of wall-bounded cases, six vector sweeps lose at 1024^2 (61 against 55)
-// and win at 2048^2 (154 against 187), hence the larger bound there.
+// below (a sweep at 512^2 4.7 -> 5.7).
 constexpr long VEC_ROWS_AUTO = 1L << 20;
-constexpr long VEC_ROWS_AUTO_WALL_SWEEPS = 1L << 21;
 bool vec_rows_on(const fugu_ctx* c, std::initializer_list<const void*> ps, long auto_min = VEC_ROWS_AUTO) {
   const int m = c->prm.vec_rows;
   if (m < 0 || (m == 0 && c->n < auto_min)) return false;
@@ -746,29 +747,80 @@ dim3 vec_grid(const Geo& g) {
   return dim3((g.P + cols - 1) / cols, (g.R + VEC_TY - 1) / VEC_TY);
 }
 
-// damped-Jacobi smoother: n sweeps of solve_helmholtz_{u,v} in place on sol
+// Whether n Jacobi sweeps of a wall-bounded case take the vectorised kernel, a
+// launch per sweep, instead of k_smooth_tile, and from which box size on.  B200,
+// us, vector / tile: one sweep 4.3 / 5.9 at 256^2 (FP32) and 69 / 118 at 2048^2
+// (FP64), two 5.4 / 6.3 and 90 / 129; three 9.6 / 6.6 at 256^2, 22 / 28 at
+// 1024^2; six 15.8 / 7.9 at 256^2, 142 / 132 at 2048^2 (FP64 268 / 255).
+constexpr long vec_wall_sweeps(int n_sweeps) {
+  return n_sweeps <= 2 ? 0L : n_sweeps == 3 ? VEC_ROWS_AUTO : LONG_MAX;
+}
+
+// The launches of `passes` passes on k_smooth_tile (passes at most ring per
+// launch).  The ring costs redundant faces (a tile of 64 x 32 regions keeps
+// 60 x 26 faces at ring 2, 52 x 18 at 6, 40 x 6 at 12), so: 2 or 4 where that
+// is enough, 12 where its CTAs still run side by side, one per SM (12 passes
+// at 128^2, FP32, us: one launch 7.8, two 10.1; at 256^2, two waves, 14.6 and
+// 10.2), else 6 (12 passes at 512^2 / 2048^2: 20 / 173 with ring 6, 23 / 190
+// with 4, 38 / 260 with 2).
+int smooth_ring(const fugu_ctx* c, int passes) {
+  if (passes <= 4) return passes <= 2 ? 2 : 4;
+  return passes > 6 && smooth_ctas(c->g, 12) <= c->nsm ? 12 : 6;
+}
+
+// smoother: n sweeps of solve_helmholtz_{u,v} in place on sol; zero: sol counts
+// as zero on entry and need not be
 template <typename T>
 void helmholtz(fugu_ctx* c, bool is_u, T* sol, T* tmp, const T* rhs, const CoefBufs<T>& cb,
-               const SolveOpt& o, double dt, int n_sweeps, const int* active) {
+               const SolveOpt& o, double dt, int n_sweeps, bool zero, const int* active) {
   Box b = box_launch(c->g);
   T* cur = sol;
   T* nxt = tmp;
   const T* pen = o.pen ? (is_u ? cb.pen_u : cb.pen_v) : nullptr;
-  if (c->prm.pcd_smoother == 1 && !c->g.px && !c->g.py) {
-    // red-black SOR, both colours of a sweep in one launch, alternating
-    // between sol and tmp (extension)
+  const T* rho = is_u ? cb.rho_u : cb.rho_v;
+  const bool sor = c->prm.pcd_smoother == 1, walls = !c->g.px && !c->g.py;
+  const bool vec = !sor && vec_rows_on(c, {sol, tmp, rhs, rho, cb.kappa, cb.zeta, cb.eta, pen},
+                                       walls ? vec_wall_sweeps(n_sweeps) : VEC_ROWS_AUTO);
+  // one sweep of FP64 SOR where k_smooth_tile's CTAs (one per SM at its
+  // registers) take several waves: the smaller tiles (512^2 9.6 against 12.0 us)
+  if (sor && walls && sizeof(T) == 8 && n_sweeps == 1 && smooth_ctas(c->g, 2) > c->nsm) {
+    if (zero) CK(cudaMemsetAsync(sol, 0, sizeof(T) * c->n, c->s));
     const dim3 grid((c->g.P + RB_TX - 1) / RB_TX, (c->g.R + RB_TY - 1) / RB_TY);
-    for (int s = 0; s < n_sweeps; ++s) {
-      k_rbsor_sweep<T><<<grid, RB_TPB, 0, c->s>>>(c->g, is_u ? 0 : 1, cur, nxt, rhs, is_u ? cb.rho_u : cb.rho_v,
-                                                  cb.kappa, cb.zeta, cb.eta, pen, T(dt), T(c->prm.pcd_sor_omega),
-                                                  active);
-      CKL("k_rbsor_sweep");
-      std::swap(cur, nxt);
+    k_rbsor_sweep<T><<<grid, RB_TPB, 0, c->s>>>(c->g, is_u ? 0 : 1, sol, tmp, rhs, rho, cb.kappa, cb.zeta, cb.eta, pen,
+                                                T(dt), T(c->prm.pcd_sor_omega), active);
+    CKL("k_rbsor_sweep");
+    CK(cudaMemcpyAsync(sol, tmp, sizeof(T) * c->n, cudaMemcpyDeviceToDevice, c->s));
+    return;
+  }
+  if (walls && !vec && n_sweeps > 0) {
+    // several passes per launch, alternating between sol and tmp
+    const int passes = sor ? 2 * n_sweeps : n_sweeps, ring = smooth_ring(c, passes);
+    const int nl = (passes + ring - 1) / ring;
+    SmoothArgs<T> a{};
+    a.g = c->g;
+    a.rhs = rhs; a.rho = rho; a.kap = cb.kappa; a.zeta = cb.zeta; a.eta = cb.eta; a.pen = pen;
+    a.dt = T(dt); a.om = T(sor ? c->prm.pcd_sor_omega : c->prm.jacobi_omega);
+    a.active = active;
+    if (zero) {  // read nothing, and let the last launch write sol
+      cur = nullptr;
+      nxt = nl & 1 ? sol : tmp;
+    }
+    for (int l = 0; l < nl; ++l) {
+      a.passes = std::min(ring, passes - l * ring);
+      a.uin = cur;
+      a.uout = nxt;
+      void* args[] = {&a};
+      CK(cudaLaunchKernel(smooth_fn<T>(sor ? SMOOTH_RBSOR : SMOOTH_JACOBI, is_u ? 0 : 1, ring), smooth_grid(c->g, ring),
+                          dim3(ST_TPB), args, 0, c->s));
+      CKL("k_smooth_tile");
+      cur = nxt;
+      nxt = cur == sol ? tmp : sol;
     }
     if (cur != sol) CK(cudaMemcpyAsync(sol, cur, sizeof(T) * c->n, cudaMemcpyDeviceToDevice, c->s));
     return;
   }
-  if (c->prm.pcd_smoother == 1) {  // red-black SOR in place, one launch per colour (periodic cases)
+  if (zero) CK(cudaMemsetAsync(sol, 0, sizeof(T) * c->n, c->s));
+  if (sor) {  // red-black SOR in place, one launch per colour (periodic cases)
     for (int s = 0; s < n_sweeps; ++s)
       for (int col = 0; col < 2; ++col) {
         halo(c, sol, is_u ? K_U : K_V, active);
@@ -782,10 +834,7 @@ void helmholtz(fugu_ctx* c, bool is_u, T* sol, T* tmp, const T* rhs, const CoefB
       }
     return;
   }
-  const T* rho = is_u ? cb.rho_u : cb.rho_v;
-  const bool walls = !c->g.px && !c->g.py;
-  if (vec_rows_on(c, {sol, tmp, rhs, rho, cb.kappa, cb.zeta, cb.eta, pen},
-                  walls ? VEC_ROWS_AUTO_WALL_SWEEPS : VEC_ROWS_AUTO)) {
+  if (vec) {
     // one sweep per launch, VW faces per thread, alternating buffers
     const dim3 grid = vec_grid<T>(c->g);
     for (int s = 0; s < n_sweeps; ++s) {
@@ -794,21 +843,6 @@ void helmholtz(fugu_ctx* c, bool is_u, T* sol, T* tmp, const T* rhs, const CoefB
                                                                cb.zeta, cb.eta, pen, T(dt), T(c->prm.jacobi_omega),
                                                                active);
       CKL("k_jacobi_vec");
-      std::swap(cur, nxt);
-    }
-    if (cur != sol) CK(cudaMemcpyAsync(sol, cur, sizeof(T) * c->n, cudaMemcpyDeviceToDevice, c->s));
-    return;
-  }
-  if (!c->g.px && !c->g.py) {
-    // up to JM_K sweeps per launch on staged tiles, alternating between sol
-    // and tmp
-    const dim3 grid((c->g.P + JM_TX - 1) / JM_TX, (c->g.R + JM_TY - 1) / JM_TY);
-    for (int s = 0; s < n_sweeps; s += JM_K) {
-      const int k = std::min(JM_K, n_sweeps - s);
-      k_jacobi_multi<T><<<grid, JM_TPB, sizeof(JmSmem<T>), c->s>>>(
-          c->g, is_u ? 0 : 1, k, cur, nxt, rhs, is_u ? cb.rho_u : cb.rho_v, cb.kappa, cb.zeta, cb.eta, pen, T(dt),
-          T(c->prm.jacobi_omega), active);
-      CKL("k_jacobi_multi");
       std::swap(cur, nxt);
     }
     if (cur != sol) CK(cudaMemcpyAsync(sol, cur, sizeof(T) * c->n, cudaMemcpyDeviceToDevice, c->s));
@@ -834,10 +868,9 @@ void pcd(fugu_ctx* c, KrylovWork<T>& w, const CoefBufs<T>& cb, const SolveOpt& o
          double dt, const int* active) {
   PcdWork<T>& pw = w.pcd;
   Box b = box_launch(c->g);
-  // r = zero; phi_p = zero (mod_pcd_precond.f90:44-47).  Plain memsets run
-  // even after an exit; the output of an exited iteration is never read.
-  CK(cudaMemsetAsync(r.base, 0, sizeof(T) * 3 * c->n, c->s));
-  CK(cudaMemsetAsync(pw.phi, 0, sizeof(T) * c->n, c->s));
+  // r = zero; phi_p = zero (mod_pcd_precond.f90:44-47): pcg() and helmholtz()
+  // take them as zero, and k_pcd_schur writes all of r_p.  The output of an
+  // exited iteration is never read.
   pcg<T>(c, w.pcg, pw.phi, z.p, c->prm.pcg_tol, c->pcg_cap_cur > 0 ? c->pcg_cap_cur : c->prm.pcg_max_iter, true,
          active);
   halo(c, pw.phi, K_CELL, active);
@@ -858,14 +891,14 @@ void pcd(fugu_ctx* c, KrylovWork<T>& w, const CoefBufs<T>& cb, const SolveOpt& o
     k_pcd_zwork<T><<<b.grid, b.block, 0, c->s>>>(c->g, z.u, z.v, r.p, pw.zuw, pw.zvw, active);
   CKL("k_pcd_zwork");
   const int sweeps = c->pcd_sweeps_cur > 0 ? c->pcd_sweeps_cur : c->prm.pcd_sweeps;
-  helmholtz<T>(c, false, r.v, pw.tmp, pw.zvw, cb, o, dt, sweeps, active);
+  helmholtz<T>(c, false, r.v, pw.tmp, pw.zvw, cb, o, dt, sweeps, true, active);
   halo(c, r.v, K_V, active);
   if (vec)
     k_pcd_cross_vec<T><<<vg, vb, 0, c->s>>>(c->g, cb.eta, r.v, pw.zuw, active);
   else
     k_pcd_cross<T><<<b.grid, b.block, 0, c->s>>>(c->g, cb.eta, r.v, pw.zuw, active);
   CKL("k_pcd_cross");
-  helmholtz<T>(c, true, r.u, pw.tmp, pw.zuw, cb, o, dt, sweeps, active);
+  helmholtz<T>(c, true, r.u, pw.tmp, pw.zuw, cb, o, dt, sweeps, true, active);
   halo(c, r.u, K_U, active);
 }
 
@@ -1784,11 +1817,6 @@ void create(fugu_ctx* c) {
     x.sum = dalloc<ulonglong2>(c, 2L * x.nslots * GX_NV);
     x.halo = dalloc<unsigned long long>(c, 4L * x.nslots * x.halo_words);
   }
-  // the multi-sweep Jacobi tiles of FP64 need more than the default 48 KB
-  CK(cudaFuncSetAttribute((const void*)k_jacobi_multi<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)sizeof(JmSmem<double>)));
-  CK(cudaFuncSetAttribute((const void*)k_jacobi_multi<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)sizeof(JmSmem<float>)));
   const char* env = std::getenv("FUGU_PCG");
   if (env && std::strcmp(env, "cluster") == 0 && !(c->pcgc[0].ok && c->pcgc[1].ok))
     throw ApiError{FUGU_EINVAL, "FUGU_PCG=cluster but this grid does not fit a thread-block cluster"};
@@ -2623,7 +2651,7 @@ int helm_entry(fugu_ctx* c, bool is_u, double* sol, const double* rhs, const dou
     else cb.pen_v = upk(c, 6, pen, K_V);
     SolveOpt o;
     o.pen = pen != nullptr;
-    helmholtz<double>(c, is_u, ds, S(c, 7), dr, cb, o, dt, n_sweeps, nullptr);
+    helmholtz<double>(c, is_u, ds, S(c, 7), dr, cb, o, dt, n_sweeps, false, nullptr);
     down(c, sol, ds, kind);
     sync(c);
   });

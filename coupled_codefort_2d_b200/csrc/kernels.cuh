@@ -914,7 +914,9 @@ __global__ void __launch_bounds__(VEC_TX * VEC_TY)
 // neighbouring tiles of the same launch write theirs: in place, it could read
 // a value its neighbour has already updated.  Callers alternate the buffers
 // and copy back after an odd number of sweeps.  A periodic case refreshes its
-// ghosts between the two colours, so it keeps the two launches.
+// ghosts between the two colours, so it keeps the two launches.  A lone case
+// runs k_smooth_tile (smooth_tile.cuh) wherever that is faster; the lockstep
+// batch runs these tiles.
 constexpr int RB_TX = 32, RB_TY = 16;
 constexpr int RB_SX = RB_TX + 4, RB_SY = RB_TY + 4;  // with the ring of two
 constexpr int RB_CX = RB_TX + 2, RB_CY = RB_TY + 2;  // with the ring of one
@@ -1025,8 +1027,8 @@ __global__ void __launch_bounds__(RB_TPB) k_rbsor_sweep(Geo g, int comp, const T
 // takes the formula with its operand order (owned faces), the right-hand side
 // (wall faces) or keeps its value (other elements), as in k_jacobi_u/v.  So
 // nsw sweeps give the bits of nsw k_jacobi_u/v launches, reading and writing
-// each array once.  Periodic cases refresh their halo between sweeps and
-// keep the one-sweep launches.
+// each array once.  The solver runs k_smooth_tile (smooth_tile.cuh); rowbench
+// times this one beside the one-sweep kernels.
 constexpr int JM_TX = 32, JM_TY = 16, JM_K = 6, JM_TPB = 256;
 constexpr int JM_SX = JM_TX + 16, JM_SY = JM_TY + 2 * JM_K;            // staged values
 constexpr int JM_CX = JM_TX + 2 * (JM_K - 1), JM_CY = JM_TY + 2 * (JM_K - 1);  // coefficients
