@@ -350,7 +350,8 @@ void halo(fugu_ctx* c, T* a, int kind, const int* active = nullptr) {
 template <typename T>
 void vbcs(fugu_ctx* c, T* u, T* v, double lid, const int* active = nullptr) {
   if (c->g.px && c->g.py) return;
-  k_velocity_bcs<T><<<1, 1024, 0, c->s>>>(c->g, u, v, T(lid), active);
+  const int n = 2 * (c->g.nx + c->g.ny + 10);  // a thread per row and side, per column and side
+  k_velocity_bcs<T><<<(n + VBC_TPB - 1) / VBC_TPB, VBC_TPB, 0, c->s>>>(c->g, u, v, T(lid), active);
   CKL("k_velocity_bcs");
 }
 

@@ -266,7 +266,7 @@ struct LsHalo {
   }
 };
 
-// wall BCs (k_velocity_bcs): of the state (lid: the step's, when final) or of Z_j
+// wall BCs (vbcs_body, the values of k_velocity_bcs): of the state (lid: the step's, when final) or of Z_j
 template <typename T>
 struct LsVbcs {
   int buf, j, final_lid;
