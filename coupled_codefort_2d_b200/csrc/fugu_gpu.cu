@@ -192,7 +192,21 @@ struct fugu_ctx {
   PcgOut* pcg_out = nullptr;
   int* svof_iters = nullptr;
   int* svof_status = nullptr;
-  // pinned host mirrors
+  // one block of pinned host memory: the mirrors below, then the staging area
+  // of the host arrays (stage)
+  unsigned char* pinned = nullptr;
+  struct Stage {
+    unsigned char* p = nullptr;
+    size_t cap = 0, at = 0;
+    bool hold = false;  // moves wait for the end of a batch (UpBatch)
+    StageArgs in;       // host-to-device moves not yet launched
+    struct Down {       // device-to-host moves launched, not yet copied out
+      double* host;
+      const unsigned char* from;
+      size_t bytes;
+    };
+    std::vector<Down> out;
+  } stage;
   KState* h_ks = nullptr;
   double* h_sc = nullptr;
   PcgOut* h_pcg = nullptr;
@@ -310,29 +324,115 @@ int kind_of_field(int f) {
   }
 }
 
-// Fortran-layout host array <-> uniform device box (strided 2-D copies)
-void copy_kind(fugu_ctx* c, double* dev, const double* host, int kind, bool h2d, double* hostw = nullptr) {
+// Fortran-layout host array <-> uniform device box.  A strided copy of pageable
+// memory is a driver call of 10-15 us and more, during which the device waits.
+// Arrays of up to STAGE_FIELD bytes go through the context's pinned staging
+// area instead, copied by the CPU on one side and by k_stage, which
+// several arrays share, over the bus on the other; sync() hands out what
+// came down.  B200, us, copies / staged: a 32^2 operator call with its 17
+// transfers 240 / 74, the four calls of a 256^2 transport step with 12 transfers
+// 1126 / 876, a 64 x 128 whole-state step with 30 transfers 7505 / 6841.
+// Larger ones keep the driver's copy, which overlaps its own staging.
+constexpr size_t STAGE_FIELD = 1 << 20, STAGE_CAP = 4 << 20;
+
+// launch the pending host-to-device moves
+void stage_flush(fugu_ctx* c) {
+  StageArgs& a = c->stage.in;
+  if (!a.n) return;
+  k_stage<<<stage_grid(a), STAGE_TPB, 0, c->s>>>(a);
+  a.n = 0;
+  CKL("k_stage");
+}
+// wait for the stream and hand out the arrays that came down
+void sync(fugu_ctx* c) {
+  stage_flush(c);
+  CK(cudaStreamSynchronize(c->s));
+  for (const auto& d : c->stage.out) std::memcpy(d.host, d.from, d.bytes);
+  c->stage.out.clear();
+  c->stage.at = 0;
+}
+// room for an array in the staging area, or nullptr (too large)
+unsigned char* stage_room(fugu_ctx* c, size_t bytes) {
+  auto& s = c->stage;
+  if (bytes > STAGE_FIELD || bytes > s.cap) return nullptr;
+  if (s.at + bytes > s.cap) sync(c);
+  unsigned char* p = s.p + s.at;
+  s.at += (bytes + 255) / 256 * 256;
+  return p;
+}
+// several up() in one launch, at the end of its scope
+struct UpBatch {
+  fugu_ctx* c;
+  bool outer;
+  explicit UpBatch(fugu_ctx* cc) : c(cc), outer(!cc->stage.hold) { c->stage.hold = true; }
+  void done() {
+    if (!outer) return;
+    c->stage.hold = false;
+    stage_flush(c);
+  }
+};
+void up(fugu_ctx* c, double* dev, const double* host, int kind) {
+  if (!host) throw ApiError{FUGU_EINVAL, "NULL host array"};
   const Geo& g = c->g;
   int i0, i1, j0, j1;
   g.extent(kind, i0, i1, j0, j1);
   const size_t w = (size_t)(i1 - i0 + 1), h = (size_t)(j1 - j0 + 1);
   double* d = dev + g.at(i0, j0);
-  if (h2d)
+  unsigned char* p = stage_room(c, sizeof(double) * w * h);
+  if (!p) {
     CK(cudaMemcpy2DAsync(d, sizeof(double) * g.P, host, sizeof(double) * w, sizeof(double) * w, h,
                          cudaMemcpyHostToDevice, c->s));
-  else
-    CK(cudaMemcpy2DAsync(hostw, sizeof(double) * w, d, sizeof(double) * g.P, sizeof(double) * w, h,
-                         cudaMemcpyDeviceToHost, c->s));
+    return;
+  }
+  std::memcpy(p, host, sizeof(double) * w * h);
+  StageArgs& a = c->stage.in;
+  a.m[a.n++] = {d, reinterpret_cast<double*>(p), (int)w, (int)h, g.P};
+  a.down = 0;
+  if (!c->stage.hold || a.n == STAGE_MOVES) stage_flush(c);
 }
-void up(fugu_ctx* c, double* dev, const double* host, int kind) {
-  if (!host) throw ApiError{FUGU_EINVAL, "NULL host array"};
-  copy_kind(c, dev, host, kind, true);
+struct DownField {
+  double* host;
+  const double* dev;
+  int kind;
+};
+// null host arrays are skipped
+void down(fugu_ctx* c, const DownField* fs, int nf) {
+  stage_flush(c);
+  StageArgs a;
+  a.n = 0;
+  a.down = 1;
+  auto launch = [&] {
+    if (!a.n) return;
+    k_stage<<<stage_grid(a), STAGE_TPB, 0, c->s>>>(a);
+    a.n = 0;
+    CKL("k_stage");
+  };
+  for (int k = 0; k < nf; ++k) {
+    const DownField& f = fs[k];
+    if (!f.host) continue;
+    const Geo& g = c->g;
+    int i0, i1, j0, j1;
+    g.extent(f.kind, i0, i1, j0, j1);
+    const size_t w = (size_t)(i1 - i0 + 1), h = (size_t)(j1 - j0 + 1), bytes = sizeof(double) * w * h;
+    double* d = const_cast<double*>(f.dev) + g.at(i0, j0);
+    if (c->stage.at + bytes > c->stage.cap) launch();  // stage_room() is about to sync
+    unsigned char* p = stage_room(c, bytes);
+    if (!p) {
+      CK(cudaMemcpy2DAsync(f.host, sizeof(double) * w, d, sizeof(double) * g.P, sizeof(double) * w, h,
+                           cudaMemcpyDeviceToHost, c->s));
+      continue;
+    }
+    a.m[a.n++] = {d, reinterpret_cast<double*>(p), (int)w, (int)h, g.P};
+    c->stage.out.push_back({f.host, p, bytes});
+    if (a.n == STAGE_MOVES) launch();
+  }
+  launch();
 }
 void down(fugu_ctx* c, double* host, const double* dev, int kind) {
   if (!host) throw ApiError{FUGU_EINVAL, "NULL host array"};
-  copy_kind(c, (double*)dev, nullptr, kind, false, host);
+  const DownField f{host, dev, kind};
+  down(c, &f, 1);
 }
-void sync(fugu_ctx* c) { CK(cudaStreamSynchronize(c->s)); }
 
 int grid1d(fugu_ctx* c, long n) {
   long b = (n + 255) / 256;
@@ -1765,10 +1865,10 @@ int coop_grid(const void* fn, int tpb, int nsm, long work, int max_ctas) {
 
 void create(fugu_ctx* c) {
   CK(cudaSetDevice(c->device));
-  cudaDeviceProp prop;
-  CK(cudaGetDeviceProperties(&prop, c->device));
-  if (!prop.cooperativeLaunch) throw ApiError{FUGU_ECUDA, "device lacks cooperative launch"};
-  c->nsm = prop.multiProcessorCount;
+  int coop = 0;  // (single attributes: the whole property set takes 2.5 ms)
+  CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
+  if (!coop) throw ApiError{FUGU_ECUDA, "device lacks cooperative launch"};
+  CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device));
   CK(cudaStreamCreateWithFlags(&c->s, cudaStreamNonBlocking));
   c->g = make_geo(c->prm);
   c->n = c->g.n();
@@ -1829,10 +1929,19 @@ void create(fugu_ctx* c) {
   c->pcg_out = dalloc<PcgOut>(c, 1);
   c->svof_iters = dalloc<int>(c, 1);
   c->svof_status = dalloc<int>(c, 1);
-  CK(cudaMallocHost(&c->h_ks, sizeof(KState)));
-  CK(cudaMallocHost(&c->h_sc, sizeof(double) * NSLOTS));
-  CK(cudaMallocHost(&c->h_pcg, sizeof(PcgOut)));
-  CK(cudaMallocHost(&c->h_int, sizeof(int) * 8));
+  {
+    auto up256 = [](size_t n) { return (n + 255) / 256 * 256; };
+    const size_t a = up256(sizeof(KState)), b = a + up256(sizeof(double) * NSLOTS), d = b + up256(sizeof(PcgOut)),
+                 e = d + up256(sizeof(int) * 8);
+    // room for the two dozen arrays of a whole-state call, at most STAGE_CAP
+    c->stage.cap = std::min(STAGE_CAP, 24 * up256(sizeof(double) * (size_t)(c->prm.nx + 5) * (c->prm.ny + 5)));
+    CK(cudaMallocHost(&c->pinned, e + c->stage.cap));
+    c->h_ks = reinterpret_cast<KState*>(c->pinned);
+    c->h_sc = reinterpret_cast<double*>(c->pinned + a);
+    c->h_pcg = reinterpret_cast<PcgOut*>(c->pinned + b);
+    c->h_int = reinterpret_cast<int*>(c->pinned + d);
+    c->stage.p = c->pinned + e;
+  }
   const double one = 1.0;
   CK(cudaMemcpyAsync(c->sc + S_ONE, &one, sizeof(double), cudaMemcpyHostToDevice, c->s));
   sync(c);
@@ -1855,10 +1964,7 @@ void destroy(fugu_ctx* c) {
   for (auto& pr : c->kr_graphs)
     for (auto& sg : pr) drop(sg);
   for (void* p : c->allocs) cudaFree(p);
-  if (c->h_ks) cudaFreeHost(c->h_ks);
-  if (c->h_sc) cudaFreeHost(c->h_sc);
-  if (c->h_pcg) cudaFreeHost(c->h_pcg);
-  if (c->h_int) cudaFreeHost(c->h_int);
+  if (c->pinned) cudaFreeHost(c->pinned);
   if (c->s) cudaStreamDestroy(c->s);
   delete c;
 }
@@ -1869,7 +1975,12 @@ int guard(fugu_ctx* c, F fn) {
   if (!c) return FUGU_EINVAL;
   try {
     cudaSetDevice(c->device);
+    c->stage.in.n = 0;  // of a call that ended in an error
+    c->stage.hold = false;
+    c->stage.out.clear();
     fn();
+    stage_flush(c);
+    if (!c->stage.out.empty()) sync(c);
     return FUGU_OK;
   } catch (const CudaError& e) {
     c->err = std::string(e.what) + ": " + cudaGetErrorString(e.e);
@@ -2025,14 +2136,18 @@ int fugu_advance_coupled_step(fugu_ctx* c, double* u_vel, double* v_vel, double*
     if (o->has_penalty && (!phi_s_u || !phi_s_v)) throw ApiError{FUGU_EINVAL, "penalty without mask"};
     double* in[] = {u_vel, v_vel, p_field, c_field, u_prev, v_prev, rho_c, rho_u, rho_v,
                     kappa, zeta, eta, kappa_curv, f_sigma_u, f_sigma_v};
+    UpBatch batch(c);
     for (int i = 0; i < 15; ++i) up(c, c->f[i], in[i], kind_of_field(i));
     if (o->has_penalty) {
       up(c, c->f[FUGU_F_PHI_S_U], phi_s_u, K_U);
       up(c, c->f[FUGU_F_PHI_S_V], phi_s_v, K_V);
     }
+    batch.done();
     if (st) std::memset(st, 0, sizeof(*st));
     step(c, dt, step_idx, o, st);
-    for (int i = 0; i < 15; ++i) down(c, in[i], c->f[i], kind_of_field(i));
+    DownField out[15];
+    for (int i = 0; i < 15; ++i) out[i] = {in[i], c->f[i], kind_of_field(i)};
+    down(c, out, 15);
     sync(c);
   });
 }
@@ -2194,6 +2309,7 @@ CoefBufs<double> up_coefs(fugu_ctx* c, const double* u_adv, const double* v_adv,
                           const double* eta, const double* pen_u, const double* pen_v, const double* mdu,
                           const double* mdv) {
   CoefBufs<double> b;
+  UpBatch batch(c);
   b.u_adv = upk(c, 4, u_adv, K_U);
   b.v_adv = upk(c, 5, v_adv, K_V);
   b.rho_c = upk(c, 6, rho_c, K_CELL);
@@ -2206,17 +2322,19 @@ CoefBufs<double> up_coefs(fugu_ctx* c, const double* u_adv, const double* v_adv,
   b.pen_v = upk(c, 13, pen_v, K_V);
   b.mdu = upk(c, 14, mdu, K_U);
   b.mdv = upk(c, 15, mdv, K_V);
+  batch.done();
   return b;
 }
 void up_trip(fugu_ctx* c, Trip<double> t, const double* u, const double* v, const double* p) {
+  UpBatch batch(c);
   up(c, t.u, u, K_U);
   up(c, t.v, v, K_V);
   up(c, t.p, p, K_CELL);
+  batch.done();
 }
 void down_trip(fugu_ctx* c, Trip<double> t, double* u, double* v, double* p) {
-  if (u) down(c, u, t.u, K_U);
-  if (v) down(c, v, t.v, K_V);
-  if (p) down(c, p, t.p, K_CELL);
+  const DownField f[] = {{u, t.u, K_U}, {v, t.v, K_V}, {p, t.p, K_CELL}};
+  down(c, f, 3);
 }
 
 // colour period of the stencil probe along one direction: 5 on a wall-bounded
@@ -2568,11 +2686,9 @@ void step_vjp(fugu_ctx* c, double dt, int step_idx, const fugu_step_opts* o, con
   k_axpby<<<g1, 256, 0, c->s>>>(n, w.b_u0, 1.0, w.b_u0, 1.0, w.b_up1);
   k_axpby<<<g1, 256, 0, c->s>>>(n, w.b_v0, 1.0, w.b_v0, 1.0, w.b_vp1);
   CKL("k_axpby");
-  down(c, bar_in[0], w.b_u0, K_U);
-  down(c, bar_in[1], w.b_v0, K_V);
-  down(c, bar_in[2], w.b_c0, K_CELL);
-  down(c, bar_in[3], w.b_up0, K_U);
-  down(c, bar_in[4], w.b_vp0, K_V);
+  const DownField bar[] = {{bar_in[0], w.b_u0, K_U}, {bar_in[1], w.b_v0, K_V}, {bar_in[2], w.b_c0, K_CELL},
+                           {bar_in[3], w.b_up0, K_U}, {bar_in[4], w.b_vp0, K_V}};
+  down(c, bar, 5);
   collect(c, nullptr);  // the adjoint SVOF's barrier status
   sync(c);
   if (st_out) {

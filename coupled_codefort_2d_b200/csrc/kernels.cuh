@@ -72,6 +72,43 @@ __global__ void k_halo(Geo g, T* a, int kind, const int* active) {
   halo_body<T>(g, a, kind);
 }
 
+// ------------------------------------------------------- host array staging
+// Copies between pinned host memory (an array's rows without padding) and the
+// device's padded rows, one array per grid row, four elements per thread in
+// flight: a read over the bus takes 1-2 us, so a few hundred threads per array
+// cover small arrays in one round trip.  Bus-bound for large ones.
+constexpr int STAGE_MOVES = 24, STAGE_TPB = 256, STAGE_U = 4;
+struct StageMove {
+  double* dev;   // first element of the box's part
+  double* host;  // pinned
+  int w, h, pitch;
+};
+struct StageArgs {
+  int n = 0, down = 0;  // down: device to host
+  StageMove m[STAGE_MOVES];
+};
+inline dim3 stage_grid(const StageArgs& a) {
+  long most = 1;
+  for (int k = 0; k < a.n; ++k) most = a.m[k].w * (long)a.m[k].h > most ? a.m[k].w * (long)a.m[k].h : most;
+  return dim3((unsigned)((most + STAGE_TPB * STAGE_U - 1) / (STAGE_TPB * STAGE_U)), (unsigned)a.n);
+}
+__global__ void __launch_bounds__(STAGE_TPB) k_stage(const __grid_constant__ StageArgs a) {
+  const StageMove m = a.m[blockIdx.y];
+  const int n = m.w * m.h, q0 = blockIdx.x * (STAGE_TPB * STAGE_U) + threadIdx.x;
+  double v[STAGE_U];
+  auto dev = [&](int q) { return m.dev + (long)(q / m.w) * m.pitch + q % m.w; };
+#pragma unroll
+  for (int e = 0; e < STAGE_U; ++e) {
+    const int q = q0 + e * STAGE_TPB;
+    if (q < n) v[e] = a.down ? *dev(q) : m.host[q];
+  }
+#pragma unroll
+  for (int e = 0; e < STAGE_U; ++e) {
+    const int q = q0 + e * STAGE_TPB;
+    if (q < n) *(a.down ? m.host + q : dev(q)) = v[e];
+  }
+}
+
 // ------------------------------------------------------------ velocity BCs
 // apply_velocity_bcs, mod_operators.f90:254-333: west, east, south, north in
 // that order (each phase reads what the previous one wrote at the corners).
