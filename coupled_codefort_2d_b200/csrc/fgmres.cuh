@@ -12,6 +12,7 @@
 // like the BiCGStab recurrences do.
 #pragma once
 
+#include "pcg_exchange.cuh"
 #include "scalars.cuh"
 
 namespace fugu {
@@ -38,7 +39,9 @@ enum FgOp {
   FG_ROTATE,    // H[j+1, j] = |w|, Givens rotations, g, rel, exit test
 };
 
-__device__ inline void fg_op(int op, const double* d, int j, double tol, const FgLayout L, double* st, KState* ks) {
+// FG_BETA and FG_ROTATE by one thread, from copies of H's column j, cs and sn
+__device__ inline void fg_op(int op, const double* d, int j, double tol, const FgLayout L, double* st, KState* ks,
+                             const double* col, const double* cs, const double* sn, double gj, double beta0) {
   switch (op) {
     case FG_BETA: {
       const double beta = sqrt(d[0]);
@@ -50,35 +53,28 @@ __device__ inline void fg_op(int op, const double* d, int j, double tol, const F
       if (!(beta > 0.0)) kexit(ks, 0);
       break;
     }
-    case FG_PROJ1:
-    case FG_PROJ2:
-      for (int i = 0; i <= j; ++i) {
-        st[L.h() + i] = d[i];
-        if (op == FG_PROJ1) st[L.H(i, j)] = 0.0;
-        st[L.H(i, j)] += d[i];
-      }
-      break;
     case FG_ROTATE: {
       const double hn = sqrt(d[0]);
-      double* col = st + L.H(0, j);
-      double* cs = st + L.cs();
-      double* sn = st + L.sn();
+      double* H = st + L.H(0, j);
       double* g = st + L.g();
-      col[j + 1] = hn;
+      double b = col[0];
       for (int i = 0; i < j; ++i) {
-        const double a = col[i], b = col[i + 1];
-        col[i] = cs[i] * a + sn[i] * b;
-        col[i + 1] = -sn[i] * a + cs[i] * b;
+        const double a = b, n = col[i + 1];
+        H[i] = cs[i] * a + sn[i] * n;
+        b = -sn[i] * a + cs[i] * n;
       }
-      const double a = col[j], b = col[j + 1];
+      const double a = b;
+      b = hn;
       const double rr = sqrt(a * a + b * b);
-      cs[j] = rr > 0.0 ? a / rr : 1.0;
-      sn[j] = rr > 0.0 ? b / rr : 0.0;
-      col[j] = rr;
-      col[j + 1] = 0.0;
-      g[j + 1] = -sn[j] * g[j];
-      g[j] = cs[j] * g[j];
-      const double rel = fabs(g[j + 1]) / st[L.beta()];
+      const double c = rr > 0.0 ? a / rr : 1.0, s = rr > 0.0 ? b / rr : 0.0;
+      st[L.cs() + j] = c;
+      st[L.sn() + j] = s;
+      H[j] = rr;
+      H[j + 1] = 0.0;
+      const double gn = -s * gj;
+      g[j + 1] = gn;
+      g[j] = c * gj;
+      const double rel = fabs(gn) / beta0;
       st[L.rel()] = rel;
       st[L.inv()] = hn > 0.0 ? 1.0 / hn : 0.0;
       if (isnan(rel)) ks->nan = 1;
@@ -92,9 +88,15 @@ __device__ inline void fg_op(int op, const double* d, int j, double tol, const F
 // are chunks of MDOT_CHUNK consecutive unknowns of one grid row of one
 // component (u, v or p rows of the owned interior), so a warp reads contiguous
 // memory and maps an item to its row once.  Each CTA keeps one DD partial for
-// its vector; the last CTA merges the partials of each vector with one warp per
-// vector and runs fg_op.  Launch: grid (Gx, nvec) of MDOT_TPB threads, grid
-// row y computing the dot with V_y.
+// its vector; the last CTA merges them and does the scalar step.  Launch: grid
+// (Gx, nvec) of MDOT_TPB threads, grid row y computing the dot with V_y.
+// Latency-bound on the grids of a step: what counts is the dependent chain
+// after the products.  The last CTA's warps share the partials of a vector with
+// four loads in flight each (a norm has up to four partials per SM, and one
+// warp read them a round trip apart), H's column is updated by a thread per
+// entry, and the rotation's inputs are read beside the partials.  B200, FP32, mean us
+// of the first launches of a step under a profiler: 8.3 -> 7.9 at 64 x 128,
+// 13.9 -> 11.9 at 320 x 640.
 constexpr int MDOT_TPB = 256;
 constexpr int MDOT_CHUNK = 128;
 constexpr int MDOT_MAXV = 128;
@@ -135,8 +137,8 @@ __device__ __forceinline__ void mdot_acc(DD& acc, double x) {
 template <typename T>
 __device__ __forceinline__ void mdot_body(const MdotArgs<T>& a, int bx, int by, int Gx, int Gy) {
   constexpr int NW = MDOT_TPB / 32;
-  __shared__ DD wsum[NW];
-  __shared__ double dsum[MDOT_MAXV];
+  __shared__ DD wsum[NW], vsum[MDOT_MAXV];
+  __shared__ double dsum[1], rot[3][MDOT_MAXV + 1];
   __shared__ bool last;
   const Geo g = a.g;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -184,36 +186,68 @@ __device__ __forceinline__ void mdot_body(const MdotArgs<T>& a, int bx, int by, 
       }
     }
   }
-  for (int o = 16; o > 0; o >>= 1) acc = dd_merge(acc, dd_shfl_down(acc, o));
+  acc = rsum_warp<true, 1>(&acc);
   if (lane == 0) wsum[warp] = acc;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    DD s = wsum[0];
-    for (int k = 1; k < NW; ++k) s = dd_merge(s, wsum[k]);
-    put_partial(a.part + 2L * by * Gx, bx, s);
-    __threadfence();
-    const unsigned int t = atomicAdd(&a.ks->ticket, 1u);
-    last = (t == (unsigned int)(Gx * Gy) - 1);
+  if (warp == 0) {
+    DD s = wsum[lane & (NW - 1)];
+#pragma unroll
+    for (int o = NW / 2; o > 0; o >>= 1) s = rsum_merge<true>(s, rsum_xor<true>(s, o));
+    if (lane == 0) {
+      put_partial(a.part + 2L * by * Gx, bx, s);
+      __threadfence();
+      const unsigned int t = atomicAdd(&a.ks->ticket, 1u);
+      last = (t == (unsigned int)(Gx * Gy) - 1);
+    }
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  for (int v = warp; v < a.nvec; v += NW) {
-    const double* pv = a.part + 2L * v * Gx;
-    DD s{0.0, 0.0};
-    for (int k = lane; k < Gx; k += 32) {
-      DD q;
-      q.hi = __ldcg(pv + 2 * k);
-      q.lo = __ldcg(pv + 2 * k + 1);
-      s = dd_merge(s, q);
+  // the rotation's inputs, read beside the partials
+  const int t = threadIdx.x;
+  double gj = 0.0, beta0 = 0.0;
+  if (a.op == FG_ROTATE) {
+    for (int i = t; i <= a.j; i += MDOT_TPB) {
+      rot[0][i] = a.st[a.L.H(i, a.j)];
+      if (i < a.j) {
+        rot[1][i] = a.st[a.L.cs() + i];
+        rot[2][i] = a.st[a.L.sn() + i];
+      }
     }
-    for (int o = 16; o > 0; o >>= 1) s = dd_merge(s, dd_shfl_down(s, o));
-    if (lane == 0) dsum[v] = s.hi + s.lo;
+    gj = a.st[a.L.g() + a.j];
+    beta0 = a.st[a.L.beta()];
+  }
+  // every warp reads: wpv of them share a vector's partials, U loads in flight
+  constexpr int U = 4;
+  const int wpv = max(1, NW / a.nvec), sub = warp % wpv;
+  for (int v = warp / wpv; v < a.nvec; v += NW / wpv) {
+    const double2* pv = reinterpret_cast<const double2*>(a.part) + (long)v * Gx;
+    DD s{0.0, 0.0};
+    for (int k = sub * 32 + lane; k < Gx; k += U * 32 * wpv) {
+      double2 q[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) q[u] = k + u * 32 * wpv < Gx ? __ldcg(pv + k + u * 32 * wpv) : double2{0.0, 0.0};
+#pragma unroll
+      for (int u = 0; u < U; ++u) s = rsum_merge<true>(s, DD{q[u].x, q[u].y});
+    }
+    s = rsum_warp<true, 1>(&s);
+    if (lane == 0) vsum[v * wpv + sub] = s;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  for (int v = t; v < a.nvec; v += MDOT_TPB) {
+    DD s = vsum[v * wpv];
+    for (int k = 1; k < wpv; ++k) s = rsum_merge<true>(s, vsum[v * wpv + k]);
+    const double d = s.hi + s.lo;
+    if (v == 0) dsum[0] = d;
+    if (a.op == FG_PROJ1 || a.op == FG_PROJ2) {
+      double& h = a.st[a.L.H(v, a.j)];
+      a.st[a.L.h() + v] = d;
+      h = (a.op == FG_PROJ1 ? 0.0 : h) + d;
+    }
+  }
+  if (t == 0) {
     a.ks->ticket = 0;
-    fg_op(a.op, dsum, a.j, a.tol, a.L, a.st, a.ks);
+    fg_op(a.op, dsum, a.j, a.tol, a.L, a.st, a.ks, rot[0], rot[1], rot[2], gj, beta0);
   }
 }
 template <typename T>
