@@ -515,7 +515,7 @@ __device__ __forceinline__ void pcgr_body(const PcgResArgs<T>& a, const int rank
       }
       if (!allreduce(IC1{}, YES{}, &rz.v, red, nothing)) return gave_up();
     }
-    double rz_old = red[0], beta = 0.0;
+    double rz_old = red[0], beta = 0.0, irz = 0.0;
     for (iter = 1; iter <= a.max_iter; ++iter) {
       const T tb = T(beta);
       // p_k of the own cells and of the halo rows
@@ -550,7 +550,11 @@ __device__ __forceinline__ void pcgr_body(const PcgResArgs<T>& a, const int rank
         apply(k, pp, ap[k]);
         PCGR_E if (e < nv[k]) papd.add(double(pp[e]) * double(ap[k][e]));
       }
-      if (!allreduce(IC1{}, NO{}, &papd.v, red, nothing)) return gave_up();
+      if (!allreduce(IC1{}, NO{}, &papd.v, red, [&] {
+            irz = 1.0 / rz_old;  // for beta, off the chain from the next sums to the update
+            asm volatile("" : "+d"(irz));
+          }))
+        return gave_up();
       const double pap = red[0];
       if (fabs(pap) < 1.0e-30) break;
       const double alpha = rz_old / pap;
@@ -578,7 +582,7 @@ __device__ __forceinline__ void pcgr_body(const PcgResArgs<T>& a, const int rank
       if (!allreduce(IC2{}, YES{}, v2, red, nothing)) return gave_up();
       rr = red[0];
       if (rr < rr_maybe && sqrt(rr) / rhs_norm < a.tol) break;
-      beta = red[1] / rz_old;
+      beta = quotient(red[1], rz_old, irz);
       rz_old = red[1];
     }
   }
