@@ -27,10 +27,10 @@
 //
 // Measured on a B200, us per iteration before (k_pcg_cluster's cluster
 // barriers, k_pcg / k_pcg1's grid barriers) and now:
-//   FP64 cluster  64 x 64 3.71 -> 2.17, 128 x 128 4.16 -> 2.88, 203 x 125 4.98 -> 4.06
-//   FP64 grid     256 x 256 7.79 -> 4.55, 320 x 640 12.5 -> 6.5, 512 x 512 13.6 -> 6.7
-//   FP32 grid     320 x 640 8.50 -> 4.22, 512 x 512 9.30 -> 4.21,
-//                 768 x 768 12.8 -> 8.5, 1024 x 1024 17.0 -> 12.7
+//   FP64 cluster  64 x 64 3.73 -> 2.14, 128 x 128 4.15 -> 2.82, 203 x 125 4.98 -> 4.01
+//   FP64 grid     256 x 256 7.79 -> 4.39, 320 x 640 12.5 -> 6.05, 512 x 512 13.7 -> 6.17
+//   FP32 grid     320 x 640 8.44 -> 3.68, 512 x 512 9.29 -> 3.70,
+//                 768 x 768 12.8 -> 7.83, 1024 x 1024 17.0 -> 12.0
 #pragma once
 
 #include <type_traits>
@@ -64,7 +64,8 @@ struct PcgResArgs {
 
 // Kernel shapes: segments per thread and largest block, by the segments of
 // a CTA.  More segments per thread mean fewer warps to reduce over but a
-// longer serial part; measured on a B200 (us per iteration): FP64 in 16 CTAs,
+// longer serial part; compared on a B200 (us per iteration, with a slower merge
+// of the received sums than now): FP64 in 16 CTAs,
 // 128 x 128 (512 segments) 2 x 256 2.81, 1 x 512 2.93; 128 x 256 (1024)
 // 4 x 256 3.96, 2 x 512 4.01; FP32 over 128 CTAs, 320 x 640 (400) 2 x 256
 // 4.22, 1 x 512 4.93; 768 x 768 (1152) 3 x 512 8.5, 4 x 512 10.5.
