@@ -25,8 +25,8 @@
 // batch (k_pcg1).  FP32 in a cluster sums in plain double, where the order
 // matters, and has its own kernel (pcg_cluster.cuh).
 //
-// Measured on a B200, us per iteration before (k_pcg_cluster's cluster
-// barriers, k_pcg / k_pcg1's grid barriers) and now:
+// Measured on a B200, us per iteration before (cluster barriers, k_pcg / k_pcg1's grid
+// barriers) and now:
 //   FP64 cluster  64 x 64 3.73 -> 2.14, 128 x 128 4.15 -> 2.82, 203 x 125 4.98 -> 4.01
 //   FP64 grid     256 x 256 7.79 -> 4.39, 320 x 640 12.5 -> 6.05, 512 x 512 13.7 -> 6.17
 //   FP32 grid     320 x 640 8.44 -> 3.68, 512 x 512 9.29 -> 3.70,

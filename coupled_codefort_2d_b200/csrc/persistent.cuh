@@ -299,8 +299,9 @@ __global__ void __launch_bounds__(512) k_pcg(PcgArgs<T> a) {
 // double it is exactly phi(i,j) - mean_val of mod_subsolvers.f90:238.
 
 // The FP32 inner solve's grid-wide PCG with one grid barrier per iteration:
-// the single-reduction (Chronopoulos-Gear) arrangement of
-// pcg_cluster_body_1r, for the grids that do not fit one cluster.  With
+// the single-reduction (Chronopoulos-Gear) arrangement, for batches whose
+// cases fit no cluster and for grids beyond the resident form
+// (pcg_resident.cuh, which has these bits).  With
 // u = M^-1 r, w = A u and s = A p, an iteration is one pass over the cells,
 //   s = w + beta s,  p = u + beta p,  phi += alpha p,  r -= alpha s,
 //   u = M^-1 r,  w = A u,  and the sums (r, u), (w, u), (r, r),
