@@ -13,8 +13,8 @@
 // inside a group of sweeps goes back to the group's start (kept in the work
 // buffer and the received rows) and repeats the sweeps up to the stop, so the
 // result and the sweep count are those of one test per sweep.  The division
-// by the constant diagonal is the exact quotient (pcg_exchange.cuh; exact down
-// to the denormals).  A sweep is straight-line code: every thread sweeps CPT
+// by the constant diagonal is the exact quotient (pcg_exchange.cuh), and a
+// division where that is not exact (svofc_exact).  A sweep is straight-line code: every thread sweeps CPT
 // rows, whether they are the CTA's own, kept or padding, and a row whose
 // neighbour is not there repeats itself (at a wall that is the mirror; beyond
 // the kept rows the value is not used again before it is received anew).
@@ -42,6 +42,14 @@ struct SvofClusterArgs {
 // shared memory in doubles: two buffers of every thread's rows, and the
 // received rows [parity][bottom, top][SVOF_T]
 inline long svofc_smem_elems(int nx, int cpt) { return 2L * (SVOFC_TPB / nx) * cpt * nx + 4L * SVOF_T * nx; }
+
+// Whether quotient(num, diag, 1 / diag) is num / diag for a diag within
+// [1, 2^100]: +0 or |num| in [2^-900, 2^900), where the remainder is exact.  Not
+// for infinities, NaN, -0 and values whose remainder would underflow.
+__device__ __forceinline__ bool svofc_exact(double num) {
+  const unsigned hi = (unsigned)__double2hiint(num), w = hi * 2u;
+  return w - (123u << 21) < (1800u << 21) || (hi | (unsigned)__double2loint(num)) == 0u;
+}
 
 template <int CPT>
 __global__ void __launch_bounds__(SVOFC_TPB, 1) k_svof_cluster(SvofClusterArgs p) {
@@ -91,6 +99,7 @@ __global__ void __launch_bounds__(SVOFC_TPB, 1) k_svof_cluster(SvofClusterArgs p
   }
   cl.sync();  // the mbarriers are initialised before any push
   const double diag = a.diag, idiag = 1.0 / diag;
+  const bool usual = diag >= 1.0 && diag <= 0x1p100;
   int cur = 0;
   // one sweep; true when a cell of the thread's own rows changed by tol or more
   auto sweep = [&]() -> bool {
@@ -99,7 +108,7 @@ __global__ void __launch_bounds__(SVOFC_TPB, 1) k_svof_cluster(SvofClusterArgs p
     double* D = S0 + (cur ^ 1) * ss + at;
     double so = strip > 0 ? S[-nx] : v[0];  // the old value below
     const double nend = strip + 1 < strips ? S[CPT * nx] : v[CPT - 1];
-    unsigned big = 0u;
+    unsigned big = 0u, odd = 0u;
 #pragma unroll
     for (int c = 0; c < CPT; ++c) {
       const double old = v[c];
@@ -108,10 +117,23 @@ __global__ void __launch_bounds__(SVOFC_TPB, 1) k_svof_cluster(SvofClusterArgs p
       if (c == ctop) nn = old;
       const double num = cr[c] + a.cx * (e + w) + a.cy * (nn + so);
       const double val = quotient(num, diag, idiag);
+      const bool exact = usual && svofc_exact(num);
+      if (!exact) odd |= 1u << c;
       v[c] = val;
-      D[c * nx] = val;
+      D[c * nx] = exact ? val : num;
       if (fabs(val - old) >= a.tol) big |= 1u << c;
       so = old;
+    }
+    if (odd) {  // rarely: divide what the quotient is not exact for
+#pragma unroll 1
+      for (int c = 0; c < CPT; ++c)
+        if ((odd >> c) & 1u) D[c * nx] = D[c * nx] / diag;
+#pragma unroll
+      for (int c = 0; c < CPT; ++c)
+        if ((odd >> c) & 1u) {
+          v[c] = D[c * nx];
+          big = fabs(v[c] - S[c * nx]) >= a.tol ? big | 1u << c : big & ~(1u << c);
+        }
     }
     return (big & own) != 0u;
   };

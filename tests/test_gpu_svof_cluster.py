@@ -32,3 +32,27 @@ def test_filter_equals_the_oracle(gpu, oracle_mod, nx, ny, px, py):
             kg = ctx.svof_helmholtz_filter(c, sg, h, iters, tol)
             assert kg == ko, (iters, tol)
             np.testing.assert_array_equal(sg, so, err_msg=f"{iters} {tol}")
+
+
+@pytest.mark.parametrize("nx,ny,px,py", [(33, 29, 0, 1), (256, 250, 0, 1)])
+def test_filter_beyond_the_exact_quotient(gpu, oracle_mod, nx, ny, px, py):
+    """Infinities, NaN, denormals, -0, huge values and a diagonal beyond 2^100: the bits of a division."""
+    g = Grid(nx, ny, periodic_x=bool(px), periodic_y=bool(py))
+    o = oracle_mod.Oracle(g, two_phase_params())
+    rng = np.random.default_rng(ny)
+    c = np.asfortranarray(rng.uniform(-0.5, 1.0, g.shape("cell")))
+    marked = c.copy(order="F")
+    marked[nx // 2, ny // 2], marked[nx // 3, ny // 4] = np.inf, np.nan
+    h = 1.5 * min(g.dx, g.dy)
+    with Context(g, two_phase_params()) as ctx:
+        for field, width in [(marked, h), (c * 1e-310, h), (c * 1e-296, h), (c * 1e303, h), (c * -0.0, h),
+                             (c, 1e20 * h)]:
+            # a NaN change counts for nothing here and resets the oracle's maximum: plain counts there
+            for iters, tol in [(7, 0.0)] + [(40, 8e-3)] * (field is not marked):
+                field = np.asfortranarray(field)
+                so, sg = g.zeros("cell"), g.zeros("cell")
+                ko = o.svof(field, so, width, iters, tol)
+                assert ctx.svof_helmholtz_filter(field, sg, width, iters, tol) == ko
+                np.testing.assert_array_equal(sg, so)
+                finite = ~np.isnan(so)
+                np.testing.assert_array_equal(np.signbit(sg[finite]), np.signbit(so[finite]))
