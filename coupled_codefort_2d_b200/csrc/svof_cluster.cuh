@@ -46,7 +46,7 @@ inline long svofc_smem_elems(int nx, int cpt) { return 2L * (SVOFC_TPB / nx) * c
 // Whether quotient(num, diag, 1 / diag) is num / diag for a diag within
 // [1, 2^100]: +0 or |num| in [2^-900, 2^900), where the remainder is exact.  Not
 // for infinities, NaN, -0 and values whose remainder would underflow.  The test
-// takes about 6 % of a 256 x 256 step's transport calls (833 -> 913 us).
+// takes about 6 % of a 256 x 256 step's transport calls (two boxes: 833 us, 913 us).
 __device__ __forceinline__ bool svofc_exact(double num) {
   const unsigned hi = (unsigned)__double2hiint(num), w = hi * 2u;
   return w - (123u << 21) < (1800u << 21) || (hi | (unsigned)__double2loint(num)) == 0u;
