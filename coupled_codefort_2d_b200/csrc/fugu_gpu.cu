@@ -730,7 +730,8 @@ void prof_drain(fugu_ctx* c) {
 }
 
 // persistent PCG (solve_poisson_pressure).  phi_zero: phi counts as zero on
-// entry; its cells need not be, its ghosts are (no PCG writes those then)
+// entry; its cells need not be, its ghosts beyond walls are (no PCG writes those
+// then; fugu_set_params clears them when a direction stops being periodic)
 template <typename T>
 void pcg(fugu_ctx* c, PcgWork<T>& w, T* phi, const T* rhs, double tol, int max_iter, bool phi_zero,
          const int* active) {
@@ -2062,8 +2063,18 @@ int fugu_set_params(fugu_ctx* c, const fugu_params* p) {
     c->err = "fugu_set_params: the grid size of a context is fixed";
     return FUGU_EINVAL;
   }
+  const bool bounds = p->periodic_x != c->prm.periodic_x || p->periodic_y != c->prm.periodic_y;
   c->prm = *p;
   c->g = make_geo(*p);
+  if (bounds) {
+    // the PCD's phi has zeros beyond a wall and its PCG does not write them
+    // (pcg()), but k_halo left a periodic direction's there
+    rc = guard(c, [&] {
+      CK(cudaMemsetAsync(c->w64.pcd.phi, 0, sizeof(double) * c->n, c->s));
+      if (c->w32_ready) CK(cudaMemsetAsync(c->w32.pcd.phi, 0, sizeof(float) * c->n, c->s));
+    });
+    if (rc) return rc;
+  }
   c->pcg_cap_state = 0;  // the adaptive PCG cap and sweeps restart from their starts
   c->pcd_sweeps_state = 0;
   return FUGU_OK;
