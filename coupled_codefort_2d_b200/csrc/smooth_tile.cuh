@@ -46,15 +46,16 @@ __device__ __forceinline__ float quotient(float a, float b, float y) {
   return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
 }
 // Whether quotient(a, b, 1 / b) may be taken for a / b, its remainder exact
-// and nothing over- or underflowing: b within smooth_b, a zero or |a| in
-// [2^-80, 2^80) (FP32), [2^-480, 2^480) (FP64); not for infinities and NaN.
+// and nothing over- or underflowing: b within smooth_b, a +0 or |a| in
+// [2^-80, 2^80) (FP32), [2^-480, 2^480) (FP64); not for infinities, NaN and -0
+// (its quotient would be +0).
 __device__ __forceinline__ bool smooth_a(float a) {
-  const unsigned w = __float_as_uint(a) * 2u;
-  return w - (47u << 24) < (160u << 24) || w == 0u;
+  const unsigned u = __float_as_uint(a), w = u * 2u;
+  return w - (47u << 24) < (160u << 24) || u == 0u;
 }
 __device__ __forceinline__ bool smooth_a(double a) {
-  const unsigned w = (unsigned)__double2hiint(a) * 2u;
-  return w - (543u << 21) < (960u << 21) || (w | (unsigned)__double2loint(a)) == 0u;
+  const unsigned hi = (unsigned)__double2hiint(a), w = hi * 2u;
+  return w - (543u << 21) < (960u << 21) || (hi | (unsigned)__double2loint(a)) == 0u;
 }
 template <typename T>
 __device__ __forceinline__ bool smooth_b(T b) { return b >= T(0x1p-40) && b <= T(0x1p40); }
