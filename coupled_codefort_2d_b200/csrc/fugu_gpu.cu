@@ -601,7 +601,10 @@ void plan_pcg_cluster(fugu_ctx* c, fugu_ctx::ClusterPlan& pl) {
   const int cmax = ny < c->max_cluster ? ny : c->max_cluster;
   if constexpr (sizeof(T) == 8) {
     const long segs = (long)ny * ((nx + 1) / 2);
-    const PcgrPlan p = pcgr_plan<double>(nx, ny, (int)std::min<long>(cmax, std::max<long>(2, segs / 128)));
+    const int want = (int)std::min<long>(cmax, std::max<long>(2, segs / 128));
+    PcgrPlan p = pcgr_plan<double>(nx, ny, want);
+    if (!p.ok || p.smem > smem_cap_of(c, pcgc_fn<double>(p.shape)))
+      p = pcgr_plan<double>(nx, ny, want, PCGR_TALL, PCGR_TALL + 1);
     if (!p.ok) return;
     pl.C = p.G;
     pl.rows_per = p.rows_per;

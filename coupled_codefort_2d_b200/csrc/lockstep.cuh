@@ -729,6 +729,7 @@ const void* ls_pcg_fn(int form) {
       case 2: return (const void*)k_ls_pcg<T, 2>;
       case 3: return (const void*)k_ls_pcg<T, 3>;
       case 4: return (const void*)k_ls_pcg<T, 4>;
+      case PCGR_TALL: return (const void*)k_ls_pcg<T, PCGR_TALL>;
     }
   } else {
     switch (form) {

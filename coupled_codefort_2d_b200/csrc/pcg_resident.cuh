@@ -69,12 +69,20 @@ struct PcgResArgs {
 // 128 x 128 (512 segments) 2 x 256 2.81, 1 x 512 2.93; 128 x 256 (1024)
 // 4 x 256 3.96, 2 x 512 4.01; FP32 over 128 CTAs, 320 x 640 (400) 2 x 256
 // 4.22, 1 x 512 4.93; 768 x 768 (1152) 3 x 512 8.5, 4 x 512 10.5.
-constexpr int PCGR_SHAPES = 5;
+// PCGR_TALL is for narrow boxes in a cluster only (FP64, 4,096 cells per CTA and
+// nx odd or 4): their half-empty last segments need a fifth one per thread and
+// their rows packed coefficients.
+constexpr int PCGR_SHAPES = 5, PCGR_TALL = 5;
 struct PcgrShape {
   int seg, tpb;
 };
 __host__ __device__ constexpr PcgrShape pcgr_shape(int s) {
-  return s == 0 ? PcgrShape{1, 256} : s == 1 ? PcgrShape{2, 256} : s == 2 ? PcgrShape{4, 256} : s == 3 ? PcgrShape{3, 512} : PcgrShape{4, 512};
+  return s == 0   ? PcgrShape{1, 256}
+         : s == 1 ? PcgrShape{2, 256}
+         : s == 2 ? PcgrShape{4, 256}
+         : s == 3 ? PcgrShape{3, 512}
+         : s == 4 ? PcgrShape{4, 512}
+                  : PcgrShape{5, 512};
 }
 
 // coefficients in registers where they fit beside the vectors
@@ -89,16 +97,24 @@ __host__ __device__ inline int pcgr_pitch(int nx) {
   const int W = 16 / (int)sizeof(T);
   return ((nx + W - 1) / W + 2) * W;
 }
+// pitch of the coefficients' rows there: padded like the vector's, or (five
+// segments per thread) packed, with one vector of padding for cx's column 0
+template <typename T>
+__host__ __device__ constexpr int pcgr_pad(int seg, bool is_cx) {
+  const int W = 16 / (int)sizeof(T);
+  return seg < pcgr_shape(PCGR_TALL).seg ? 2 * W : is_cx ? W : 0;
+}
 // shared memory (elements of T): the stencil's vector with its two halo
 // rows, the received halo rows (two parities), their recurrence in the
 // single-reduction form (s, r and the inverse diagonal), and the
 // coefficients when they are not in registers
 template <typename T>
 __host__ __device__ inline long pcgr_smem_elems(int nx, int rows_per, int seg, int tpb) {
-  const long p = pcgr_pitch<T>(nx);
+  const int W = 16 / (int)sizeof(T);
+  const long p = pcgr_pitch<T>(nx), px = p - 2 * W + pcgr_pad<T>(seg, true), py = p - 2 * W + pcgr_pad<T>(seg, false);
   long n = (rows_per + 2) * p + 4 * p;
   if (sizeof(T) == 4) n += 6 * p;
-  if (!pcgr_reg_coefs<T>(seg, tpb)) n += 3 * rows_per * p + p;
+  if (!pcgr_reg_coefs<T>(seg, tpb)) n += rows_per * px + (2 * rows_per + 1) * py;
   return n;
 }
 
@@ -132,8 +148,12 @@ __device__ __forceinline__ void pcgr_body(const PcgResArgs<T>& a, const int rank
   T* hr = hs + 2 * P;
   T* hd = hr + 2 * P;
   T* cxs = ONE ? hd + 2 * P : hs;           // (only without RC) cx, cy (rows j0 - 1 ..), dinv
-  T* cys = cxs + rp * P;
-  T* dis = cys + (rp + 1) * P;
+  // their pitches and the slot of column 1
+  constexpr bool PACK = pcgr_pad<T>(SEG, false) == 0;
+  const int PX = PACK ? P - W : P, PY = PACK ? P - 2 * W : P;
+  constexpr int Y1 = PACK ? 0 : W;
+  T* cys = cxs + rp * PX;
+  T* dis = cys + (rp + 1) * PY;
   __shared__ std::conditional_t<CL, ClusterXSmem<TPB>, GridXSmem<TPB>> xs;
   auto x = [&] {
     if constexpr (CL) return ClusterX<TPB, true>(xs, rank, G);
@@ -173,14 +193,16 @@ __device__ __forceinline__ void pcgr_body(const PcgResArgs<T>& a, const int rank
       PCGR_E dg[k][e] = cE[k][e] + (e ? cE[k][e ? e - 1 : 0] : cW0[k]) + cN[k][e] + cS[k][e];
     }
   } else {
-    for (int q = tid; q < R * P; q += tpb) {
-      const int lr = q / P, i = q % P - W + 1;
+    for (int q = tid; q < R * PX; q += tpb) {
+      const int lr = q / PX, i = q % PX - W + 1;
       cxs[q] = (i >= 0 && i <= nx) ? a.cx[g.at(i, j0 + lr)] : T(0);
-      dis[q] = (i >= 1 && i <= nx) ? a.dinv[g.at(i, j0 + lr)] : T(0);
+      if constexpr (!PACK) dis[q] = (i >= 1 && i <= nx) ? a.dinv[g.at(i, j0 + lr)] : T(0);
     }
-    for (int q = tid; q < (R + 1) * P; q += tpb) {
-      const int lf = q / P - 1, i = q % P - W + 1;
+    for (int q = tid; q < (R + 1) * PY; q += tpb) {
+      const int lf = q / PY - 1, i = q % PY - Y1 + 1;
       cys[q] = (i >= 1 && i <= nx) ? a.cy[g.at(i, j0 + lf)] : T(0);
+      if constexpr (PACK)
+        if (lf >= 0) dis[q - PY] = i <= nx ? a.dinv[g.at(i, j0 + lf)] : T(0);
     }
   }
   // every slot of the stencil's vector is finite (padding is read, times a
@@ -349,11 +371,11 @@ __device__ __forceinline__ void pcgr_body(const PcgResArgs<T>& a, const int rank
     const T wv = us[c - 1], ev = us[c + nv[k]];
     T xE[W], xN[W], xS[W], xW0;
     if constexpr (!RC) {
-      const int q = sx(k, lr);
+      const int q = lr * PX + W + i0[k] - 1, qy = lr * PY + Y1 + i0[k] - 1;
       ldv(cxs + q, xE);
       xW0 = cxs[q - 1];
-      ldv(cys + q + P, xN);
-      ldv(cys + q, xS);
+      ldv(cys + qy + PY, xN);
+      ldv(cys + qy, xS);
     }
     PCGR_E {
       const T fE = RC ? cE[RC ? k : 0][e] : xE[e];
@@ -371,7 +393,7 @@ __device__ __forceinline__ void pcgr_body(const PcgResArgs<T>& a, const int rank
     if constexpr (RC) {
       PCGR_E d[e] = di[k][e];
     } else {
-      ldv(dis + sx(k, row[k]), d);
+      ldv(dis + row[k] * PY + Y1 + i0[k] - 1, d);
     }
   };
   // the halo rows' segments: f(side, index of the segment in a halo array,
@@ -628,6 +650,9 @@ const void* pcgr_fn(int shape) {
     case 2: return (const void*)k_pcg_resident<T, 2, CL>;
     case 3: return (const void*)k_pcg_resident<T, 3, CL>;
     case 4: return (const void*)k_pcg_resident<T, 4, CL>;
+    case PCGR_TALL:
+      if constexpr (CL) return (const void*)k_pcg_resident<T, PCGR_TALL, CL>;
+      break;
   }
   return nullptr;
 }
@@ -638,16 +663,16 @@ struct PcgrPlan {
   int G = 0, rows_per = 0, shape = 0, tpb = 0;
   size_t smem = 0;
 };
-// the plan for want_G CTAs (or fewer, when ny does not divide); not ok when
-// the rows do not fit a CTA's registers
+// the plan for want_G CTAs (or fewer, when ny does not divide) with the first
+// of the shapes [s0, s1) that holds a CTA's rows; not ok when none does
 template <typename T>
-PcgrPlan pcgr_plan(int nx, int ny, int want_G) {
+PcgrPlan pcgr_plan(int nx, int ny, int want_G, int s0 = 0, int s1 = PCGR_SHAPES) {
   PcgrPlan p;
   const int W = 16 / (int)sizeof(T), nseg = (nx + W - 1) / W;
   p.rows_per = (ny + want_G - 1) / want_G;
   p.G = (ny + p.rows_per - 1) / p.rows_per;
   const long segs = (long)p.rows_per * nseg;
-  for (int s = 0; s < PCGR_SHAPES && !p.ok; ++s) {
+  for (int s = s0; s < s1 && !p.ok; ++s) {
     const PcgrShape sh = pcgr_shape(s);
     if (segs > (long)sh.seg * sh.tpb) continue;
     p.shape = s;
