@@ -27,6 +27,8 @@
 
 #include <cooperative_groups.h>
 
+#include <cstddef>
+
 #include "fugu_internal.cuh"
 
 namespace fugu {
@@ -128,8 +130,8 @@ __device__ __forceinline__ bool mbar_test(unsigned bar, unsigned phase) {
 }
 
 template <int TPB>
-struct ClusterXSmem {
-  double rcv[2][CX_MAXC][4];  // received sums [parity][rank]
+struct alignas(16) ClusterXSmem {
+  double rcv[2][CX_MAXC][4];  // received sums [parity][rank]; first, for push16's 16-byte stores
   DD wp[3][TPB / 32];         // the warps' sums
   double bc[3];               // the totals
   unsigned long long mbar[2];
@@ -141,6 +143,8 @@ struct ClusterXSmem {
 template <int TPB, bool DDS>
 struct ClusterX {
   static constexpr int NP = DDS ? 2 : 1;  // doubles per sum
+  static_assert(alignof(ClusterXSmem<TPB>) >= 16 && offsetof(ClusterXSmem<TPB>, rcv) == 0,
+                "push16 stores 16 bytes at rcv[parity][rank][q * NP]");
   ClusterXSmem<TPB>& s;
   int rank, G;
   unsigned ep;
