@@ -220,6 +220,7 @@ struct fugu_ctx {
   // limits for concurrent use (a batch lowers them so many cases fit at once)
   int max_cluster = 16;  // CTAs of the cluster-resident PCG
   int max_coop = 1 << 30;  // CTAs of a grid-wide cooperative kernel
+  int max_svof = 16;       // CTAs of the SVOF filter's cluster
   bool coop_as_cluster = false;  // launch those as one cluster (max_coop <= 8)
   // Krylov iterations whose PCG is the grid-wide kernel are captured into
   // graphs as cooperative kernel nodes; cleared (for good) if a capture or an
@@ -656,13 +657,13 @@ void plan_pcg_grid(fugu_ctx* c, PcgrPlan& p) {
   if (!p.ok) cudaGetLastError();
 }
 
-// Plan the SVOF filter's cluster: about 512 cells per CTA, up to max_cluster
+// Plan the SVOF filter's cluster: about 512 cells per CTA, up to max_svof
 // CTAs, each (the last one too) with at least the SVOF_T rows its neighbours keep
 void plan_svof(fugu_ctx* c, fugu_ctx::SvofPlan& pl) {
   pl = fugu_ctx::SvofPlan{};
   const int nx = c->prm.nx, ny = c->prm.ny;
   if (nx > SVOFC_TPB) return;
-  const long want = std::min<long>(std::min(c->max_cluster, ny / SVOF_T), std::max(1L, (long)nx * ny / 512));
+  const long want = std::min<long>(std::min(c->max_svof, ny / SVOF_T), std::max(1L, (long)nx * ny / 512));
   for (int C = (int)want; C >= 1; --C) {
     const int rows_per = (ny + C - 1) / C, n = (ny + rows_per - 1) / rows_per, last = ny - (n - 1) * rows_per;
     if (last < SVOF_T) continue;
@@ -2102,8 +2103,9 @@ int fugu_profile(fugu_ctx* c, int enable, fugu_profile_stats* out) {
       out->pcg_launches = c->prof_pcg_launches;
       out->pcg_iters = c->prof_pcg_iters;
       out->pcg_cells = c->prof_pcg_cells;
-      out->pcg_grid = c->pcg_grid;
-      out->svof_grid = c->svof_grid;
+      const PcgrPlan& gp = c->pcgg[c->prm.precision == FUGU_MIXED ? 1 : 0];
+      out->pcg_grid = gp.ok ? gp.G : c->pcg_grid;
+      out->svof_grid = c->svofc.ok ? c->svofc.C : c->svof_grid;
       out->pcg_cluster_fp64 = c->pcgc[0].ok ? c->pcgc[0].C : 0;
       out->pcg_cluster_fp32 = c->pcgc[1].ok ? c->pcgc[1].C : 0;
       out->pcg_iters_timed = c->prof_pcg_iters_timed;
@@ -3496,6 +3498,7 @@ int fugu_batch_create(const fugu_params* params, int ncases, int device, const f
     c->prm = params[i];
     c->device = device;
     c->max_coop = o.max_coop ? std::min(o.max_coop, 8) : 8;
+    if (o.max_coop) c->max_svof = c->max_coop;
     c->coop_as_cluster = true;
     c->max_cluster = o.max_cluster ? o.max_cluster : 16;
     b->cases.push_back(c);

@@ -166,7 +166,9 @@ typedef struct {
   unsigned long long pcg_launches;    /* timed PCG launches                    */
   unsigned long long pcg_iters;       /* PCG iterations of all launches        */
   unsigned long long pcg_cells;       /* cells per PCG iteration (nx*ny)       */
-  int pcg_grid, svof_grid;            /* CTAs of the persistent kernels        */
+  int pcg_grid;                       /* CTAs of the PCG over the whole device */
+                                      /*   (of the precision that iterates)    */
+  int svof_grid;                      /* CTAs of the SVOF filter               */
   int pcg_cluster_fp64;               /* CTAs of the cluster-resident PCG (0:   */
   int pcg_cluster_fp32;               /*   the case fits no cluster)            */
   unsigned long long pcg_iters_timed; /* PCG iterations of the timed launches  */
@@ -386,7 +388,8 @@ typedef struct {
   int nthreads;     /* host threads stepping cases (0: hardware threads, <= ncases) */
   int max_cluster;  /* CTAs of each cluster-resident PCG, 1..16 (0: autotune)     */
   int max_coop;     /* CTAs of each grid-wide persistent kernel, launched as one  */
-                    /* thread-block cluster so that it is scheduled whole (<= 8; 0: 8) */
+                    /* thread-block cluster so that it is scheduled whole (<= 8; 0: 8, */
+                    /* and up to 16 for the SVOF filter where its rows fit a cluster)  */
   int lockstep;     /* 1: the coupled solves of all cases advance in lockstep,
                        one launch per kernel family serving every case still
                        running (work lists of (case, tile) items on the device,
