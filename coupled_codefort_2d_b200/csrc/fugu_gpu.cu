@@ -333,8 +333,16 @@ int kind_of_field(int f) {
 // came down.  B200, us, copies / staged: a 32^2 operator call with its 17
 // transfers 240 / 74, the four calls of a 256^2 transport step with 12 transfers
 // 1126 / 876, a 64 x 128 whole-state step with 30 transfers 7505 / 6841.
-// Larger ones keep the driver's copy, which overlaps its own staging.
-constexpr size_t STAGE_FIELD = 1 << 20, STAGE_CAP = 4 << 20;
+// Larger ones keep the driver's copy, which overlaps its own staging.  So do
+// page-locked arrays above STAGE_ANY, which the driver moves without the CPU: the 17
+// transfers of an operator call, copies / staged, 162 / 73 at 32^2, 306 / 236 at 128^2,
+// 451 / 435 at 192^2, 511 / 778 at 256^2, 685 / 1210 at 320^2.  The question costs 1.1 us
+// an array, so smaller ones are not asked about.
+constexpr size_t STAGE_FIELD = 1 << 20, STAGE_CAP = 4 << 20, STAGE_ANY = 256 << 10;
+// An array that comes down alone gains little by staging (pageable, copy / staged,
+// 16.3 / 18.3 at 32^2, 26.6 / 27.9 at 128^2, 40.6 / 36.7 at 190^2; page-locked 13.4 / 18.2,
+// 15.4 / 28.0, 18.4 / 34.1): up to this size it takes the driver's copy.
+constexpr size_t STAGE_LONE = 160 << 10;
 
 // launch the pending host-to-device moves
 void stage_flush(fugu_ctx* c) {
@@ -352,10 +360,18 @@ void sync(fugu_ctx* c) {
   c->stage.out.clear();
   c->stage.at = 0;
 }
-// room for an array in the staging area, or nullptr (too large)
-unsigned char* stage_room(fugu_ctx* c, size_t bytes) {
+// whether the driver knows the memory (page-locked, managed, a device's)
+bool page_locked(const void* host) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, host) == cudaSuccess) return a.type != cudaMemoryTypeUnregistered;
+  cudaGetLastError();
+  return false;
+}
+// room for a host array in the staging area, or nullptr (the driver's copy);
+// any: the size up to which nothing is asked about the array's memory
+unsigned char* stage_room(fugu_ctx* c, const void* host, size_t bytes, size_t any = STAGE_ANY) {
   auto& s = c->stage;
-  if (bytes > STAGE_FIELD || bytes > s.cap) return nullptr;
+  if (bytes > STAGE_FIELD || bytes > s.cap || (bytes > any && page_locked(host))) return nullptr;
   if (s.at + bytes > s.cap) sync(c);
   unsigned char* p = s.p + s.at;
   s.at += (bytes + 255) / 256 * 256;
@@ -379,7 +395,7 @@ void up(fugu_ctx* c, double* dev, const double* host, int kind) {
   g.extent(kind, i0, i1, j0, j1);
   const size_t w = (size_t)(i1 - i0 + 1), h = (size_t)(j1 - j0 + 1);
   double* d = dev + g.at(i0, j0);
-  unsigned char* p = stage_room(c, sizeof(double) * w * h);
+  unsigned char* p = stage_room(c, host, sizeof(double) * w * h);
   if (!p) {
     CK(cudaMemcpy2DAsync(d, sizeof(double) * g.P, host, sizeof(double) * w, sizeof(double) * w, h,
                          cudaMemcpyHostToDevice, c->s));
@@ -396,8 +412,8 @@ struct DownField {
   const double* dev;
   int kind;
 };
-// null host arrays are skipped
-void down(fugu_ctx* c, const DownField* fs, int nf) {
+// null host arrays are skipped; lone: nothing else comes down with it
+void down(fugu_ctx* c, const DownField* fs, int nf, bool lone = false) {
   stage_flush(c);
   StageArgs a;
   a.n = 0;
@@ -417,7 +433,7 @@ void down(fugu_ctx* c, const DownField* fs, int nf) {
     const size_t w = (size_t)(i1 - i0 + 1), h = (size_t)(j1 - j0 + 1), bytes = sizeof(double) * w * h;
     double* d = const_cast<double*>(f.dev) + g.at(i0, j0);
     if (c->stage.at + bytes > c->stage.cap) launch();  // stage_room() is about to sync
-    unsigned char* p = stage_room(c, bytes);
+    unsigned char* p = lone && bytes <= STAGE_LONE ? nullptr : stage_room(c, f.host, bytes, lone ? STAGE_LONE : STAGE_ANY);
     if (!p) {
       CK(cudaMemcpy2DAsync(f.host, sizeof(double) * w, d, sizeof(double) * g.P, sizeof(double) * w, h,
                            cudaMemcpyDeviceToHost, c->s));
@@ -433,6 +449,11 @@ void down(fugu_ctx* c, double* host, const double* dev, int kind) {
   if (!host) throw ApiError{FUGU_EINVAL, "NULL host array"};
   const DownField f{host, dev, kind};
   down(c, &f, 1);
+}
+void down_lone(fugu_ctx* c, double* host, const double* dev, int kind) {
+  if (!host) throw ApiError{FUGU_EINVAL, "NULL host array"};
+  const DownField f{host, dev, kind};
+  down(c, &f, 1, true);
 }
 
 int grid1d(fugu_ctx* c, long n) {
@@ -2129,7 +2150,7 @@ int fugu_upload(fugu_ctx* c, int field, const double* host) {
 int fugu_download(fugu_ctx* c, int field, double* host) {
   return guard(c, [&] {
     if (field < 0 || field >= FUGU_NUM_FIELDS) throw ApiError{FUGU_EINVAL, "bad field id"};
-    down(c, host, c->f[field], kind_of_field(field));
+    down_lone(c, host, c->f[field], kind_of_field(field));
     sync(c);
   });
 }
@@ -2218,13 +2239,13 @@ int fugu_build_cylinder_mask(fugu_ctx* c, double xc, double yc, double rad, doub
 }
 
 int fugu_halo_scalar(fugu_ctx* c, double* phi) {
-  return guard(c, [&] { upk(c, 0, phi, K_CELL); halo(c, S(c, 0), K_CELL); down(c, phi, S(c, 0), K_CELL); sync(c); });
+  return guard(c, [&] { upk(c, 0, phi, K_CELL); halo(c, S(c, 0), K_CELL); down_lone(c, phi, S(c, 0), K_CELL); sync(c); });
 }
 int fugu_halo_u(fugu_ctx* c, double* u) {
-  return guard(c, [&] { upk(c, 0, u, K_U); halo(c, S(c, 0), K_U); down(c, u, S(c, 0), K_U); sync(c); });
+  return guard(c, [&] { upk(c, 0, u, K_U); halo(c, S(c, 0), K_U); down_lone(c, u, S(c, 0), K_U); sync(c); });
 }
 int fugu_halo_v(fugu_ctx* c, double* v) {
-  return guard(c, [&] { upk(c, 0, v, K_V); halo(c, S(c, 0), K_V); down(c, v, S(c, 0), K_V); sync(c); });
+  return guard(c, [&] { upk(c, 0, v, K_V); halo(c, S(c, 0), K_V); down_lone(c, v, S(c, 0), K_V); sync(c); });
 }
 
 int fugu_compute_mixture_densities(fugu_ctx* c, const double* cf, double* rho_c, double* rho_u, double* rho_v) {
@@ -2255,7 +2276,7 @@ int fugu_op_divergence(fugu_ctx* c, const double* u, const double* v, double* di
     Box b = box_launch(c->g);
     k_op_divergence<<<b.grid, b.block, 0, c->s>>>(c->g, du, dv, S(c, 2));
     CKL("k_op_divergence");
-    down(c, div, S(c, 2), K_CELL);
+    down_lone(c, div, S(c, 2), K_CELL);
     sync(c);
   });
 }
@@ -2756,7 +2777,7 @@ int fugu_solve_poisson_pressure(fugu_ctx* c, double* phi, const double* rhs, con
     poisson_coefs<double>(c, c->w64.pcg, dru, drv);
     pcg<double>(c, c->w64.pcg, dphi, drhs, tol, max_iter, false, nullptr);
     collect(c, nullptr);
-    down(c, phi, dphi, K_CELL);
+    down_lone(c, phi, dphi, K_CELL);
     CK(cudaMemcpyAsync(c->h_pcg, c->pcg_out, sizeof(PcgOut), cudaMemcpyDeviceToHost, c->s));
     sync(c);
     if (iter_out) *iter_out = c->h_pcg->iters;
@@ -2785,7 +2806,7 @@ int helm_entry(fugu_ctx* c, bool is_u, double* sol, const double* rhs, const dou
     SolveOpt o;
     o.pen = pen != nullptr;
     helmholtz<double>(c, is_u, ds, S(c, 7), dr, cb, o, dt, n_sweeps, false, nullptr);
-    down(c, sol, ds, kind);
+    down_lone(c, sol, ds, kind);
     sync(c);
   });
 }
@@ -2941,10 +2962,12 @@ int fugu_vof_advection_tvd(fugu_ctx* c, const double* c_in, double* c_out, const
     double* dv = upk(c, 2, v, K_V);
     const bool fl = flux_x && flux_y;
     vof(c, ci, S(c, 3), du, dv, dt, fl ? S(c, 4) : nullptr, fl ? S(c, 5) : nullptr);
-    down(c, c_out, S(c, 3), K_CELL);
     if (fl) {
+      down(c, c_out, S(c, 3), K_CELL);
       down(c, flux_x, S(c, 4), K_U);
       down(c, flux_y, S(c, 5), K_V);
+    } else {
+      down_lone(c, c_out, S(c, 3), K_CELL);
     }
     sync(c);
   });
@@ -2959,7 +2982,7 @@ int fugu_svof_helmholtz_filter(fugu_ctx* c, const double* c_raw, double* c_smoot
     fugu_stats st{};
     collect(c, &st);
     if (iters_out) *iters_out = st.svof_iters;
-    down(c, c_smooth, S(c, 1), K_CELL);
+    down_lone(c, c_smooth, S(c, 1), K_CELL);
     sync(c);
   });
 }
@@ -2968,7 +2991,7 @@ int fugu_compute_interface_curvature(fugu_ctx* c, const double* c_smooth, double
   return guard(c, [&] {
     double* cs = upk(c, 0, c_smooth, K_CELL);
     curvature(c, cs, S(c, 1));
-    down(c, kappa_curv, S(c, 1), K_CELL);
+    down_lone(c, kappa_curv, S(c, 1), K_CELL);
     sync(c);
   });
 }
