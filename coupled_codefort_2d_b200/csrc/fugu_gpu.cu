@@ -149,6 +149,15 @@ struct VjpWork {
   ad::Dual *dgu = nullptr, *dgv = nullptr;
 };
 
+// A page-locked staging area for host arrays.  A context of its own has one; the
+// cases of a batch, hundreds of them perhaps, share their batch's, and a call that
+// finds it taken by another thread's call leaves its arrays to the driver's copies.
+struct StageArea {
+  unsigned char* p = nullptr;
+  size_t cap = 0;
+  std::mutex m;
+};
+
 }  // namespace
 
 struct fugu_ctx {
@@ -192,12 +201,15 @@ struct fugu_ctx {
   PcgOut* pcg_out = nullptr;
   int* svof_iters = nullptr;
   int* svof_status = nullptr;
-  // one block of pinned host memory: the mirrors below, then the staging area
-  // of the host arrays (stage)
+  // one block of pinned host memory: the mirrors below and, in a context of its
+  // own, the staging area of the host arrays
   unsigned char* pinned = nullptr;
+  StageArea own_area;
   struct Stage {
-    unsigned char* p = nullptr;
-    size_t cap = 0, at = 0;
+    StageArea* area = nullptr;  // own_area, or a batch's (null: none)
+    bool held = false;          // by the API call in progress
+    bool busy = false;          // moves since the last sync()
+    size_t at = 0;
     bool hold = false;  // moves wait for the end of a batch (UpBatch)
     StageArgs in;       // host-to-device moves not yet launched
     struct Down {       // device-to-host moves launched, not yet copied out
@@ -327,8 +339,8 @@ int kind_of_field(int f) {
 
 // Fortran-layout host array <-> uniform device box.  A strided copy of pageable
 // memory is a driver call of 10-15 us and more, during which the device waits.
-// Arrays of up to STAGE_FIELD bytes go through the context's pinned staging
-// area instead, copied by the CPU on one side and by k_stage, which
+// Arrays of up to STAGE_FIELD bytes go through a pinned staging area
+// (StageArea) instead, copied by the CPU on one side and by k_stage, which
 // several arrays share, over the bus on the other; sync() hands out what
 // came down.  B200, us, copies / staged: a 32^2 operator call with its 17
 // transfers 240 / 74, the four calls of a 256^2 transport step with 12 transfers
@@ -359,6 +371,7 @@ void sync(fugu_ctx* c) {
   for (const auto& d : c->stage.out) std::memcpy(d.host, d.from, d.bytes);
   c->stage.out.clear();
   c->stage.at = 0;
+  c->stage.busy = false;
 }
 // whether the driver knows the memory (page-locked, managed, a device's)
 bool page_locked(const void* host) {
@@ -368,15 +381,34 @@ bool page_locked(const void* host) {
   return false;
 }
 // room for a host array in the staging area, or nullptr (the driver's copy);
-// any: the size up to which nothing is asked about the array's memory
+// any: the size up to which nothing is asked about the array's memory.  The area
+// is held until the end of the API call (StageHold).
 unsigned char* stage_room(fugu_ctx* c, const void* host, size_t bytes, size_t any = STAGE_ANY) {
   auto& s = c->stage;
-  if (bytes > STAGE_FIELD || bytes > s.cap || (bytes > any && page_locked(host))) return nullptr;
-  if (s.at + bytes > s.cap) sync(c);
-  unsigned char* p = s.p + s.at;
+  if (!s.area || bytes > STAGE_FIELD || bytes > s.area->cap || (bytes > any && page_locked(host))) return nullptr;
+  if (!s.held && !s.area->m.try_lock()) return nullptr;
+  s.held = s.busy = true;
+  if (s.at + bytes > s.area->cap) {
+    sync(c);
+    s.busy = true;
+  }
+  unsigned char* p = s.area->p + s.at;
   s.at += (bytes + 255) / 256 * 256;
   return p;
 }
+// gives the staging area back when nothing on the stream uses it any more, also
+// after a call that ended in an error
+struct StageHold {
+  fugu_ctx* c;
+  ~StageHold() {
+    auto& s = c->stage;
+    if (!s.held) return;
+    if (s.busy) cudaStreamSynchronize(c->s);
+    s.busy = s.held = false;
+    s.at = 0;
+    s.area->m.unlock();
+  }
+};
 // several up() in one launch, at the end of its scope
 struct UpBatch {
   fugu_ctx* c;
@@ -432,7 +464,7 @@ void down(fugu_ctx* c, const DownField* fs, int nf, bool lone = false) {
     g.extent(f.kind, i0, i1, j0, j1);
     const size_t w = (size_t)(i1 - i0 + 1), h = (size_t)(j1 - j0 + 1), bytes = sizeof(double) * w * h;
     double* d = const_cast<double*>(f.dev) + g.at(i0, j0);
-    if (c->stage.at + bytes > c->stage.cap) launch();  // stage_room() is about to sync
+    if (c->stage.held && c->stage.at + bytes > c->stage.area->cap) launch();  // stage_room() is about to sync
     unsigned char* p = lone && bytes <= STAGE_LONE ? nullptr : stage_room(c, f.host, bytes, lone ? STAGE_LONE : STAGE_ANY);
     if (!p) {
       CK(cudaMemcpy2DAsync(f.host, sizeof(double) * w, d, sizeof(double) * g.P, sizeof(double) * w, h,
@@ -1959,14 +1991,19 @@ void create(fugu_ctx* c) {
     auto up256 = [](size_t n) { return (n + 255) / 256 * 256; };
     const size_t a = up256(sizeof(KState)), b = a + up256(sizeof(double) * NSLOTS), d = b + up256(sizeof(PcgOut)),
                  e = d + up256(sizeof(int) * 8);
-    // room for the two dozen arrays of a whole-state call, at most STAGE_CAP
-    c->stage.cap = std::min(STAGE_CAP, 24 * up256(sizeof(double) * (size_t)(c->prm.nx + 5) * (c->prm.ny + 5)));
-    CK(cudaMallocHost(&c->pinned, e + c->stage.cap));
+    size_t cap = 0;
+    if (!c->coop_as_cluster) {
+      // room for the two dozen arrays of a whole-state call, at most STAGE_CAP
+      cap = std::min(STAGE_CAP, 24 * up256(sizeof(double) * (size_t)(c->prm.nx + 5) * (c->prm.ny + 5)));
+      c->stage.area = &c->own_area;
+    }
+    CK(cudaMallocHost(&c->pinned, e + cap));
     c->h_ks = reinterpret_cast<KState*>(c->pinned);
     c->h_sc = reinterpret_cast<double*>(c->pinned + a);
     c->h_pcg = reinterpret_cast<PcgOut*>(c->pinned + b);
     c->h_int = reinterpret_cast<int*>(c->pinned + d);
-    c->stage.p = c->pinned + e;
+    c->own_area.p = c->pinned + e;
+    c->own_area.cap = cap;
   }
   const double one = 1.0;
   CK(cudaMemcpyAsync(c->sc + S_ONE, &one, sizeof(double), cudaMemcpyHostToDevice, c->s));
@@ -1999,6 +2036,7 @@ void destroy(fugu_ctx* c) {
 template <typename F>
 int guard(fugu_ctx* c, F fn) {
   if (!c) return FUGU_EINVAL;
+  StageHold hold{c};
   try {
     cudaSetDevice(c->device);
     c->stage.in.n = 0;  // of a call that ended in an error
@@ -3098,6 +3136,7 @@ struct fugu_batch {
   cudaStream_t s = nullptr;
   cudaEvent_t ev_start = nullptr;
   std::vector<cudaEvent_t> ev_case;  // per case: its stage of the run is done
+  StageArea stage;                   // the cases'
 };
 
 namespace {
@@ -3514,6 +3553,10 @@ int fugu_batch_create(const fugu_params* params, int ncases, int device, const f
   const int hw = (int)std::thread::hardware_concurrency();
   b->nthreads = o.nthreads ? o.nthreads : (hw > 0 ? hw : 8);
   if (b->nthreads > ncases) b->nthreads = ncases;
+  if (cudaSetDevice(device) == cudaSuccess && cudaMallocHost(&b->stage.p, STAGE_CAP) == cudaSuccess)
+    b->stage.cap = STAGE_CAP;
+  else
+    cudaGetLastError();  // a bad device is reported with the first case
   // autotune decisions shared by cases of the same grid, boundaries and precision
   std::map<std::array<int, 5>, int> tuned;
   for (int i = 0; i < ncases; ++i) {
@@ -3523,6 +3566,7 @@ int fugu_batch_create(const fugu_params* params, int ncases, int device, const f
     c->max_coop = o.max_coop ? std::min(o.max_coop, 8) : 8;
     if (o.max_coop) c->max_svof = c->max_coop;
     c->coop_as_cluster = true;
+    if (b->stage.cap) c->stage.area = &b->stage;
     c->max_cluster = o.max_cluster ? o.max_cluster : 16;
     b->cases.push_back(c);
     const int rc = guard(c, [&] {
@@ -3544,6 +3588,7 @@ int fugu_batch_create(const fugu_params* params, int ncases, int device, const f
       b->err = "case " + std::to_string(i) + ": " + c->err;
       fprintf(stderr, "fugu_batch_create: %s\n", b->err.c_str());
       for (fugu_ctx* x : b->cases) destroy(x);
+      if (b->stage.cap) cudaFreeHost(b->stage.p);
       delete b;
       return rc;
     }
@@ -3585,6 +3630,7 @@ void fugu_batch_destroy(fugu_batch* b) {
   }
   for (LockstepBase* ls : b->groups) delete ls;
   for (fugu_ctx* c : b->cases) destroy(c);
+  if (b->stage.cap) cudaFreeHost(b->stage.p);
   delete b;
 }
 
