@@ -1717,8 +1717,15 @@ void collect(fugu_ctx* c, fugu_stats* st) {
   CK(cudaMemcpyAsync(c->h_int + 1, c->svof_status, sizeof(int), cudaMemcpyDeviceToHost, c->s));
   CK(cudaMemcpyAsync(c->h_int + 2, &c->gs->error, sizeof(int), cudaMemcpyDeviceToHost, c->s));
   sync(c);
-  if (c->h_int[1] || c->h_int[2] || c->h_pcg->status)
+  if (c->h_int[1] || c->h_int[2] || c->h_pcg->status) {
+    const Exchange& x = c->xch;
+    if (x.epoch) {  // what the launch left there must not pass for a later one's (pcg_exchange.cuh)
+      CK(cudaMemsetAsync(x.epoch, 0, sizeof(unsigned int), c->s));
+      CK(cudaMemsetAsync(x.sum, 0, sizeof(ulonglong2) * 2 * x.nslots * GX_NV, c->s));
+      CK(cudaMemsetAsync(x.halo, 0, sizeof(unsigned long long) * 4 * x.nslots * x.halo_words, c->s));
+    }
     throw ApiError{FUGU_ETIMEOUT, "a persistent kernel's grid barrier gave up waiting"};
+  }
   if (st) {
     st->pcg_iters = (long long)c->h_pcg->total_iters;
     st->pcg_calls = (int)c->h_pcg->calls;

@@ -19,7 +19,9 @@
 // CTA sends exchange e + 2 only after it received every CTA's e + 1, which each
 // CTA sends after it has read everything of e, so nothing is overwritten
 // before all its readers are done.  The grid's numbers keep growing from
-// launch to launch (Exchange::epoch), so nothing is cleared in between.
+// launch to launch (Exchange::epoch), so nothing is cleared in between.  A launch
+// in which a wait gave up leaves words of numbers that a later one would use, and
+// a CTA that starts late may add some, so the host clears the buffers after it.
 //
 // Every wait is bounded: after its limit of polls, or when another CTA has
 // flagged an error, allreduce returns false and the kernel unwinds.
@@ -331,7 +333,7 @@ struct GridX {
     __syncthreads();
   }
   // by one thread, when every CTA has taken part in an exchange of the launch
-  __device__ __forceinline__ void finish(unsigned skip) { *x.epoch = ep + skip; }
+  __device__ __forceinline__ void finish() { *x.epoch = ep; }
   __device__ __forceinline__ unsigned parity() const { return ep & 1u; }
   __device__ __forceinline__ unsigned long long* outbox(int cta, int side) const {
     return x.halo + (((long)(ep & 1u) * x.nslots + cta) * 2 + side) * x.halo_words;

@@ -275,7 +275,6 @@ __device__ __forceinline__ void pcgr_body(const PcgResArgs<T>& a, const int rank
   auto gave_up = [&]() {
     if (tid == 0) a.out->status = 1;
     if constexpr (CL) x.abandon();
-    else if (rank == 0 && tid == 0) x.finish(2u * (unsigned)a.max_iter + 16u);
   };
   using IC1 = std::integral_constant<int, 1>;
   using IC2 = std::integral_constant<int, 2>;
@@ -334,7 +333,7 @@ __device__ __forceinline__ void pcgr_body(const PcgResArgs<T>& a, const int rank
       a.out->iters = 0;
       a.out->res = 0.0;
       a.out->calls += 1;
-      if constexpr (!CL) x.finish(0);
+      if constexpr (!CL) x.finish();
     }
     return leave();
   }
@@ -624,7 +623,7 @@ __device__ __forceinline__ void pcgr_body(const PcgResArgs<T>& a, const int rank
     a.out->total_iters += (unsigned long long)it;
     if (a.timed) a.out->timed_iters += (unsigned long long)it;
     a.out->calls += 1;
-    if constexpr (!CL) x.finish(0);
+    if constexpr (!CL) x.finish();
   }
   leave();
 #undef PCGR_SEGS
