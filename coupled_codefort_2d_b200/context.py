@@ -109,6 +109,11 @@ class Context:
         FUGU_ETIMEOUT (``fugu_test_arm_barrier_timeout``)."""
         self._ck(self.L.fugu_test_arm_barrier_timeout(self.h, int(spin_limit)))
 
+    def arm_cluster_timeout(self, spin_limit: int = 1000):
+        """The same for the next launch of this context that exchanges within a
+        thread-block cluster (``fugu_test_arm_cluster_timeout``)."""
+        self._ck(self.L.fugu_test_arm_cluster_timeout(self.h, int(spin_limit)))
+
     def _f(self, a, kind):
         return ptr(as_fortran(a, self.g, kind))
 

@@ -25,6 +25,7 @@
 #include <string>
 #include <thread>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "fugu_gpu.h"
@@ -229,6 +230,7 @@ struct fugu_ctx {
   // failure-detection test hook: > 0 arms the next grid-wide PCG launch to
   // wait for one CTA too many and give up after this many polls
   unsigned int test_spin_limit = 0;
+  unsigned int test_cluster_limit = 0;  // the same for the next cluster launch
   // limits for concurrent use (a batch lowers them so many cases fit at once)
   int max_cluster = 16;  // CTAs of the cluster-resident PCG
   int max_coop = 1 << 30;  // CTAs of a grid-wide cooperative kernel
@@ -786,6 +788,13 @@ void prof_drain(fugu_ctx* c) {
   c->ev_pcg.clear();
 }
 
+// the bound of the next cluster launch's waits: the armed test's, once and not in
+// a capture, or the usual one
+CxLimit cluster_limit(fugu_ctx* c) {
+  if (c->capturing || !c->test_cluster_limit) return CxLimit{0u, 0u};
+  return CxLimit{std::exchange(c->test_cluster_limit, 0u), 16u};
+}
+
 // persistent PCG (solve_poisson_pressure).  phi_zero: phi counts as zero on
 // entry; its cells need not be, its ghosts beyond walls are (no PCG writes those
 // then; fugu_set_params clears them when a direction stops being periodic)
@@ -843,11 +852,13 @@ void pcg(fugu_ctx* c, PcgWork<T>& w, T* phi, const T* rhs, double tol, int max_i
     } else {
       PcgClusterArgs ca{};
       void* args[] = {&ra};
+      ra.wait = cluster_limit(c);
       if constexpr (sizeof(T) == 4) {
         ca.g = ra.g;
         ca.rhs = ra.rhs; ca.cx = ra.cx; ca.cy = ra.cy; ca.dinv = ra.dinv; ca.phi = ra.phi;
         ca.out = ra.out; ca.active = ra.active; ca.tol = ra.tol; ca.max_iter = ra.max_iter;
         ca.phi_zero = ra.phi_zero; ca.rows_per = ra.rows_per; ca.timed = ra.timed;
+        ca.wait = ra.wait;
         args[0] = &ca;
       }
       cudaLaunchAttribute at[1];
@@ -1658,7 +1669,7 @@ void vof(fugu_ctx* c, const double* cin, double* cout, const double* u, const do
 // the filter's kernel on the context's stream
 void svof_launch(fugu_ctx* c, SvofArgs& a) {
   if (c->svofc.ok) {
-    SvofClusterArgs ca{a, c->svofc.rows_per};
+    SvofClusterArgs ca{a, c->svofc.rows_per, cluster_limit(c)};
     void* args[] = {&ca};
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = cluster_cfg(c->svofc.C, SVOFC_TPB, c->svofc.smem, c->s, at);
@@ -3900,5 +3911,10 @@ extern "C" int fugu_test_arm_barrier_timeout(fugu_ctx* ctx, unsigned int spin_li
   if (spin_limit == 0) return FUGU_EINVAL;
   if (ctx) ctx->test_spin_limit = spin_limit;
   else na_test_spin_limit.store(spin_limit);
+  return FUGU_OK;
+}
+extern "C" int fugu_test_arm_cluster_timeout(fugu_ctx* ctx, unsigned int spin_limit) {
+  if (!ctx || spin_limit == 0) return FUGU_EINVAL;
+  ctx->test_cluster_limit = spin_limit;
   return FUGU_OK;
 }

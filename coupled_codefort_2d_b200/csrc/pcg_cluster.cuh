@@ -64,6 +64,7 @@ struct PcgClusterArgs {
   int phi_zero;
   int rows_per;  // rows of every CTA but possibly the last
   int timed;     // the launch is timed: add its iterations to out->timed_iters
+  CxLimit wait;  // k_pcg_column's waits
 };
 
 // ------------------------------------------------------------ column strips
@@ -109,7 +110,7 @@ __device__ __forceinline__ void pcg_column_body(const PcgClusterArgs& a, const i
   T* dis = cys + (rp + 1) * nx;
   T* phs = dis + rp * nx;
   __shared__ ClusterXSmem<PCGC_TPB> xs;
-  ClusterX<PCGC_TPB, false> x(xs, rank, C);
+  ClusterX<PCGC_TPB, false> x(xs, rank, C, a.wait);
 
 #define COL_CELLS _Pragma("unroll") for (int c = 0; c < CPT; ++c) if (c < nr)
   T phi_r[RC ? CPT : 1], r_r[CPT], u_r[RC ? CPT : 1], w_r[CPT], p_r[CPT], s_r[CPT];

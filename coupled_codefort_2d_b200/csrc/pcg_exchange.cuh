@@ -131,6 +131,13 @@ __device__ __forceinline__ bool mbar_test(unsigned bar, unsigned phase) {
   return ok != 0;
 }
 
+// the bound of a cluster's waits, in polls (0: FUGU_SPIN_LIMIT); the
+// failure-detection test lowers it and expects bytes that nobody sends
+struct CxLimit {
+  unsigned int spin_limit, extra_bytes;
+  __device__ __forceinline__ unsigned polls() const { return spin_limit ? spin_limit : FUGU_SPIN_LIMIT; }
+};
+
 template <int TPB>
 struct alignas(16) ClusterXSmem {
   double rcv[2][CX_MAXC][4];  // received sums [parity][rank]; first, for push16's 16-byte stores
@@ -149,8 +156,9 @@ struct ClusterX {
                 "push16 stores 16 bytes at rcv[parity][rank][q * NP]");
   ClusterXSmem<TPB>& s;
   int rank, G;
-  unsigned ep;
-  __device__ __forceinline__ ClusterX(ClusterXSmem<TPB>& sm, int r, int g) : s(sm), rank(r), G(g), ep(0) {}
+  unsigned ep, lim, extra;
+  __device__ __forceinline__ ClusterX(ClusterXSmem<TPB>& sm, int r, int g, CxLimit l)
+      : s(sm), rank(r), G(g), ep(0), lim(l.polls()), extra(l.extra_bytes) {}
   __device__ __forceinline__ void start() {
     if (threadIdx.x == 0) {
       s.fail = 0;
@@ -176,7 +184,7 @@ struct ClusterX {
     const unsigned par = ep & 1u, mb = smem_u32(&s.mbar[par]);
     if (tid == 0)
       asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(mb),
-                   "r"((unsigned)(G * NV * NP * 8) + halo_bytes)
+                   "r"((unsigned)(G * NV * NP * 8) + halo_bytes + extra)
                    : "memory");
     {
       const DD t = rsum_warp<DDS, NV>(v);
@@ -209,7 +217,7 @@ struct ClusterX {
     if (warp < NV) {
       unsigned spins = 0;
       while (!mbar_test(mb, (ep >> 1) & 1u))
-        if (++spins > FUGU_SPIN_LIMIT) {
+        if (++spins > lim) {
           ok = false;
           break;
         }

@@ -60,6 +60,7 @@ struct PcgResArgs {
   int* err;                 // the launch's error flag (GridSync::error)
   unsigned int spin_limit;  // 0: FUGU_SPIN_LIMIT / 16 (a poll is a global round trip)
   int extra_arrivals;       // failure-detection test: wait for a slot nobody writes
+  CxLimit wait;             // cluster exchange only
 };
 
 // Kernel shapes: segments per thread and largest block, by the segments of
@@ -156,7 +157,7 @@ __device__ __forceinline__ void pcgr_body(const PcgResArgs<T>& a, const int rank
   T* dis = cys + (rp + 1) * PY;
   __shared__ std::conditional_t<CL, ClusterXSmem<TPB>, GridXSmem<TPB>> xs;
   auto x = [&] {
-    if constexpr (CL) return ClusterX<TPB, true>(xs, rank, G);
+    if constexpr (CL) return ClusterX<TPB, true>(xs, rank, G, a.wait);
     else return GridX<TPB>(xs, a.x, rank, G, a.extra_arrivals, a.spin_limit, a.err);
   }();
 

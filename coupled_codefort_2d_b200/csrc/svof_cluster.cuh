@@ -38,6 +38,7 @@ constexpr int SVOF_T = 4;  // sweeps per exchange
 struct SvofClusterArgs {
   SvofArgs a;
   int rows_per;  // rows of every CTA but possibly the last (at least SVOF_T each)
+  CxLimit wait;
 };
 // shared memory in doubles: two buffers of every thread's rows, and the
 // received rows [parity][bottom, top][SVOF_T]
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(SVOFC_TPB, 1) k_svof_cluster(SvofClusterArgs p
     const unsigned par = ep & 1u, mb = smem_u32(&mbar[par]);
     if (t == 0)
       asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(mb),
-                   "r"((unsigned)(4 * C) + (last ? 0u : (unsigned)(((int)has_bot + (int)has_top) * SVOF_T * nx * 8)))
+                   "r"((unsigned)(4 * C) + p.wait.extra_bytes + (last ? 0u : (unsigned)(((int)has_bot + (int)has_top) * SVOF_T * nx * 8)))
                    : "memory");
     if (!last) {
       const unsigned hp = smem_u32(hw + par * 2 * SVOF_T * nx);
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(SVOFC_TPB, 1) k_svof_cluster(SvofClusterArgs p
       unsigned spins = 0;
       bool ok = true;
       while (!mbar_test(mb, (ep >> 1) & 1u))
-        if (++spins > FUGU_SPIN_LIMIT) {
+        if (++spins > p.wait.polls()) {
           ok = false;
           break;
         }

@@ -490,6 +490,11 @@ int fugu_solve_poisson_pressure_noalloc(const fugu_params* p, void* stream, doub
  * would run, and a launch inside a CUDA-graph capture is never armed.
  * One-shot: later launches run normally. */
 int fugu_test_arm_barrier_timeout(fugu_ctx* ctx, unsigned int spin_limit);
+/* The same for the next launch of ctx that exchanges within a thread-block
+ * cluster (the cluster-resident PCG on column strips or in FP64, the SVOF
+ * filter): each of its CTAs waits for bytes that no CTA sends and gives up
+ * after spin_limit polls (>= 1). */
+int fugu_test_arm_cluster_timeout(fugu_ctx* ctx, unsigned int spin_limit);
 
 #ifdef __cplusplus
 }
