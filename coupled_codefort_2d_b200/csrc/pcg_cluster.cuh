@@ -21,12 +21,12 @@
 //     (the east, west and strip-end neighbours).  The rows just outside the
 //     CTA belong to single columns of its edge threads: each receives w of its
 //     halo cell with the sums and repeats the cell's s, r and u itself.
-//   k_pcg_cluster_lean  strips of up to 32 cells in a batch, such as 320 x 512,
-//     with the reference's recurrence: five register arrays of 32 cells do
-//     not fit, so z is recomputed from r and p_k lives in shared memory.
-//     Halo rows of z and p are pushed into the neighbouring CTAs and the
-//     CTAs meet at hardware cluster barriers.  15.2 us per iteration at
-//     320 x 384 on a B200.
+//   k_pcg_cluster_lean  strips of 17 to 32 cells, alone or in a batch, such as
+//     320 x 384, 400 x 400 or 200 x 600, with the reference's recurrence: five
+//     register arrays of 32 cells do not fit, so z is recomputed from r and p_k
+//     lives in shared memory.  Halo rows of z and p are pushed into the
+//     neighbouring CTAs and the CTAs meet at hardware cluster barriers.  15.2 us
+//     per iteration at 320 x 384 on a B200.
 //
 // k_pcg_column is bound by the latency chain of its iteration and, at 4,096
 // cells per CTA, by the conversions to double of the three products per cell

@@ -9,7 +9,9 @@
 //   cluster  every CTA pushes its sums into the shared memory of all CTAs of
 //            its thread-block cluster and its boundary rows into its
 //            neighbours' (st.async), and waits on its own mbarrier for the
-//            bytes it expects.  About 200 cycles on a B200 for 16 CTAs.
+//            bytes it expects.  On a B200 a bare exchange of 8 bytes takes 357
+//            cycles between 16 CTAs (236 between 2), an all-reduce of 16 x 512
+//            threads 1,028 (FP32, one sum) to 2,063 (FP64, two sums).
 //   grid     8-byte words in global memory hold four bytes of payload and the
 //            32-bit number of the exchange, so a reader that sees the
 //            expected number has the payload too (an aligned 8-byte access is

@@ -21,8 +21,8 @@
 // What bounds it: the FP64 operations of the rows of a SM (11 per cell and
 // sweep at 64 per cycle) and the barrier between sweeps.
 // us on a B200 before and now (sweeps to the step's tolerance): 64 x 128 (71)
-// 252 -> 47, 128 x 256 (73) 270 -> 90, 256 x 256 (115) 420 -> 225, 192 x 384
-// (73) 273 -> 186; a batch's cases, which ran the grid-wide kernel on 8 CTAs,
+// 238 -> 43, 128 x 256 (73) 249 -> 85, 256 x 256 (115) 392 -> 240, 192 x 384
+// (73) 249 -> 177; a batch's cases, which ran the grid-wide kernel on 8 CTAs,
 // gain more.  256 x 512 needs 24 rows per thread, which spill (528 against
 // 319), so it and wider grids keep the grid-wide kernel.
 #pragma once
@@ -46,8 +46,9 @@ inline long svofc_smem_elems(int nx, int cpt) { return 2L * (SVOFC_TPB / nx) * c
 
 // Whether quotient(num, diag, 1 / diag) is num / diag for a diag within
 // [1, 2^100]: +0 or |num| in [2^-900, 2^900), where the remainder is exact.  Not
-// for infinities, NaN, -0 and values whose remainder would underflow.  The test
-// takes about 6 % of a 256 x 256 step's transport calls (two boxes: 833 us, 913 us).
+// for infinities, NaN, -0 and values whose remainder would underflow.  Of the
+// filter's time the test takes 4 us at 64 x 128 and 28 us at 256 x 256 (212 us
+// without it), 9-13 %.
 __device__ __forceinline__ bool svofc_exact(double num) {
   const unsigned hi = (unsigned)__double2hiint(num), w = hi * 2u;
   return w - (123u << 21) < (1800u << 21) || (hi | (unsigned)__double2loint(num)) == 0u;

@@ -65,7 +65,8 @@ class Params:
     pcd_visc_scale: float = 0.0
     # 1: the damped-Jacobi sweeps and the PCD's Schur, residual and cross
     # steps take 16-byte vector accesses (same results); -1 never; 0 for
-    # boxes of at least 2^20 points (the sweeps of wall-bounded cases 2^21)
+    # boxes of at least 2^20 points (the Jacobi sweeps of wall-bounded cases: one or
+    # two at any size, three from 2^20, more never)
     vec_rows: int = 0
 
     def with_(self, **kw) -> "Params":

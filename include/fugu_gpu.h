@@ -113,8 +113,11 @@ typedef struct {
                                  vector accesses, 16 / sizeof(real) elements
                                  of a row per thread (same results): 1 on,
                                  -1 off, 0 on for boxes of >= 2^20 points
-                                 (large grids, where they stream HBM; the
-                                 sweeps of wall-bounded cases from 2^21)    */
+                                 (large grids, where they stream HBM); the
+                                 Jacobi sweeps of wall-bounded cases by
+                                 their number instead: one or two at any
+                                 size, three from 2^20 points, four and
+                                 more never (several per launch on tiles)   */
 } fugu_params;
 
 /* Optional arguments of advance_coupled_step (src/mod_solver_coupled.f90:137-160):
@@ -382,7 +385,10 @@ int fugu_read_checkpoint(fugu_ctx* ctx, const char* path, int* step, double* t);
  * at once as fit.  With max_cluster = 0 the CTAs of each case's
  * cluster-resident PCG are autotuned at creation: per distinct (grid,
  * boundaries, precision) every feasible size in {2, 4, 8, 16} is timed on
- * the device and the least CTAs x time per iteration wins. */
+ * the device and the least CTAs x time per iteration wins; in FP32, sizes that
+ * give a thread more than 8 cells are left out where another gives fewer.  The
+ * cases share one 4 MB page-locked staging area for their host arrays (a context
+ * of its own has one). */
 typedef struct fugu_batch fugu_batch;
 typedef struct {
   int nthreads;     /* host threads stepping cases (0: hardware threads, <= ncases) */
