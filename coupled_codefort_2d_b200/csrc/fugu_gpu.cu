@@ -353,10 +353,26 @@ int kind_of_field(int f) {
 // 451 / 435 at 192^2, 511 / 778 at 256^2, 685 / 1210 at 320^2.  The question costs 1.1 us
 // an array, so smaller ones are not asked about.
 constexpr size_t STAGE_FIELD = 1 << 20, STAGE_CAP = 4 << 20, STAGE_ANY = 256 << 10;
-// An array that comes down alone gains little by staging (pageable, copy / staged,
-// 16.3 / 18.3 at 32^2, 26.6 / 27.9 at 128^2, 40.6 / 36.7 at 190^2; page-locked 13.4 / 18.2,
-// 15.4 / 28.0, 18.4 / 34.1): up to this size it takes the driver's copy.
+// Who else moves with an array: others in the same launch, other transfers and
+// kernels of a routine, or nothing (fugu_upload, fugu_download).
+enum Moves { MOVES_SHARED, MOVES_ROUTINE, MOVES_ALONE };
+// Whether an array goes up by the driver's copy for its shape: the copy costs by the
+// row, staging does not, and the copy overlaps its own staging with the bus.  Pageable,
+// copy / staged.  The 17 transfers of an operator call, 600 KB in 36 rows 1006 / 910, 900 KB
+// in 36 1290 / 1329, in 132 1400 / 1323.  A divergence (two up, one down), 240 KB in 20 rows
+// 83 / 74, 400 KB in 20 108 / 116, in 68 115 / 114, 600 KB in 20 149 / 171, in 68 169 / 172, in
+// 132 197 / 171.  One array up alone, 64 KB in 20 rows 25 / 20, 120 KB in 20 22 / 24, in 36 27 /
+// 23, 900 KB in 20 64 / 71.
+bool up_by_copy(size_t bytes, size_t rows, Moves m) {
+  constexpr size_t K = 1 << 10;
+  if (m == MOVES_SHARED) return bytes > 768 * K && rows <= 128;
+  return (bytes > (m == MOVES_ALONE ? 100 : 320) * K && rows <= 24) || (bytes > 512 * K && rows <= 96);
+}
+// And whether an array that comes down alone does: up to this size in boxes that are not
+// tall (pageable 16.3 / 18.3 at 32^2, 26.6 / 27.9 at 128^2, but 56 / 25 at 55 x 256; page-locked
+// 13.4 / 18.2, 15.4 / 28.0).
 constexpr size_t STAGE_LONE = 160 << 10;
+bool down_by_copy(size_t bytes, size_t cols, size_t rows) { return bytes <= STAGE_LONE && 2 * cols >= rows; }
 
 // launch the pending host-to-device moves
 void stage_flush(fugu_ctx* c) {
@@ -422,20 +438,22 @@ struct UpBatch {
     stage_flush(c);
   }
 };
-void up(fugu_ctx* c, double* dev, const double* host, int kind) {
+void up(fugu_ctx* c, double* dev, const double* host, int kind, bool alone = false) {
   if (!host) throw ApiError{FUGU_EINVAL, "NULL host array"};
   const Geo& g = c->g;
   int i0, i1, j0, j1;
   g.extent(kind, i0, i1, j0, j1);
   const size_t w = (size_t)(i1 - i0 + 1), h = (size_t)(j1 - j0 + 1);
   double* d = dev + g.at(i0, j0);
-  unsigned char* p = stage_room(c, host, sizeof(double) * w * h);
+  const size_t bytes = sizeof(double) * w * h;
+  const Moves m = c->stage.hold ? MOVES_SHARED : alone ? MOVES_ALONE : MOVES_ROUTINE;
+  unsigned char* p = up_by_copy(bytes, h, m) ? nullptr : stage_room(c, host, bytes);
   if (!p) {
     CK(cudaMemcpy2DAsync(d, sizeof(double) * g.P, host, sizeof(double) * w, sizeof(double) * w, h,
                          cudaMemcpyHostToDevice, c->s));
     return;
   }
-  std::memcpy(p, host, sizeof(double) * w * h);
+  std::memcpy(p, host, bytes);
   StageArgs& a = c->stage.in;
   a.m[a.n++] = {d, reinterpret_cast<double*>(p), (int)w, (int)h, g.P};
   a.down = 0;
@@ -446,8 +464,8 @@ struct DownField {
   const double* dev;
   int kind;
 };
-// null host arrays are skipped; lone: nothing else comes down with it
-void down(fugu_ctx* c, const DownField* fs, int nf, bool lone = false) {
+// null host arrays are skipped
+void down(fugu_ctx* c, const DownField* fs, int nf, Moves m = MOVES_ROUTINE) {
   stage_flush(c);
   StageArgs a;
   a.n = 0;
@@ -467,7 +485,9 @@ void down(fugu_ctx* c, const DownField* fs, int nf, bool lone = false) {
     const size_t w = (size_t)(i1 - i0 + 1), h = (size_t)(j1 - j0 + 1), bytes = sizeof(double) * w * h;
     double* d = const_cast<double*>(f.dev) + g.at(i0, j0);
     if (c->stage.held && c->stage.at + bytes > c->stage.area->cap) launch();  // stage_room() is about to sync
-    unsigned char* p = lone && bytes <= STAGE_LONE ? nullptr : stage_room(c, f.host, bytes, lone ? STAGE_LONE : STAGE_ANY);
+    unsigned char* p = nullptr;
+    if (m != MOVES_ALONE) p = stage_room(c, f.host, bytes);
+    else if (!down_by_copy(bytes, w, h)) p = stage_room(c, f.host, bytes, STAGE_LONE);
     if (!p) {
       CK(cudaMemcpy2DAsync(f.host, sizeof(double) * w, d, sizeof(double) * g.P, sizeof(double) * w, h,
                            cudaMemcpyDeviceToHost, c->s));
@@ -479,17 +499,11 @@ void down(fugu_ctx* c, const DownField* fs, int nf, bool lone = false) {
   }
   launch();
 }
-void down(fugu_ctx* c, double* host, const double* dev, int kind) {
+void down(fugu_ctx* c, double* host, const double* dev, int kind, Moves m = MOVES_ROUTINE) {
   if (!host) throw ApiError{FUGU_EINVAL, "NULL host array"};
   const DownField f{host, dev, kind};
-  down(c, &f, 1);
+  down(c, &f, 1, m);
 }
-void down_lone(fugu_ctx* c, double* host, const double* dev, int kind) {
-  if (!host) throw ApiError{FUGU_EINVAL, "NULL host array"};
-  const DownField f{host, dev, kind};
-  down(c, &f, 1, true);
-}
-
 int grid1d(fugu_ctx* c, long n) {
   long b = (n + 255) / 256;
   long cap = (long)c->nsm * 8;
@@ -2199,14 +2213,14 @@ int fugu_profile(fugu_ctx* c, int enable, fugu_profile_stats* out) {
 int fugu_upload(fugu_ctx* c, int field, const double* host) {
   return guard(c, [&] {
     if (field < 0 || field >= FUGU_NUM_FIELDS) throw ApiError{FUGU_EINVAL, "bad field id"};
-    up(c, c->f[field], host, kind_of_field(field));
+    up(c, c->f[field], host, kind_of_field(field), true);
     sync(c);
   });
 }
 int fugu_download(fugu_ctx* c, int field, double* host) {
   return guard(c, [&] {
     if (field < 0 || field >= FUGU_NUM_FIELDS) throw ApiError{FUGU_EINVAL, "bad field id"};
-    down_lone(c, host, c->f[field], kind_of_field(field));
+    down(c, host, c->f[field], kind_of_field(field), MOVES_ALONE);
     sync(c);
   });
 }
@@ -2295,13 +2309,13 @@ int fugu_build_cylinder_mask(fugu_ctx* c, double xc, double yc, double rad, doub
 }
 
 int fugu_halo_scalar(fugu_ctx* c, double* phi) {
-  return guard(c, [&] { upk(c, 0, phi, K_CELL); halo(c, S(c, 0), K_CELL); down_lone(c, phi, S(c, 0), K_CELL); sync(c); });
+  return guard(c, [&] { upk(c, 0, phi, K_CELL); halo(c, S(c, 0), K_CELL); down(c, phi, S(c, 0), K_CELL); sync(c); });
 }
 int fugu_halo_u(fugu_ctx* c, double* u) {
-  return guard(c, [&] { upk(c, 0, u, K_U); halo(c, S(c, 0), K_U); down_lone(c, u, S(c, 0), K_U); sync(c); });
+  return guard(c, [&] { upk(c, 0, u, K_U); halo(c, S(c, 0), K_U); down(c, u, S(c, 0), K_U); sync(c); });
 }
 int fugu_halo_v(fugu_ctx* c, double* v) {
-  return guard(c, [&] { upk(c, 0, v, K_V); halo(c, S(c, 0), K_V); down_lone(c, v, S(c, 0), K_V); sync(c); });
+  return guard(c, [&] { upk(c, 0, v, K_V); halo(c, S(c, 0), K_V); down(c, v, S(c, 0), K_V); sync(c); });
 }
 
 int fugu_compute_mixture_densities(fugu_ctx* c, const double* cf, double* rho_c, double* rho_u, double* rho_v) {
@@ -2332,7 +2346,7 @@ int fugu_op_divergence(fugu_ctx* c, const double* u, const double* v, double* di
     Box b = box_launch(c->g);
     k_op_divergence<<<b.grid, b.block, 0, c->s>>>(c->g, du, dv, S(c, 2));
     CKL("k_op_divergence");
-    down_lone(c, div, S(c, 2), K_CELL);
+    down(c, div, S(c, 2), K_CELL);
     sync(c);
   });
 }
@@ -2833,7 +2847,7 @@ int fugu_solve_poisson_pressure(fugu_ctx* c, double* phi, const double* rhs, con
     poisson_coefs<double>(c, c->w64.pcg, dru, drv);
     pcg<double>(c, c->w64.pcg, dphi, drhs, tol, max_iter, false, nullptr);
     collect(c, nullptr);
-    down_lone(c, phi, dphi, K_CELL);
+    down(c, phi, dphi, K_CELL);
     CK(cudaMemcpyAsync(c->h_pcg, c->pcg_out, sizeof(PcgOut), cudaMemcpyDeviceToHost, c->s));
     sync(c);
     if (iter_out) *iter_out = c->h_pcg->iters;
@@ -2862,7 +2876,7 @@ int helm_entry(fugu_ctx* c, bool is_u, double* sol, const double* rhs, const dou
     SolveOpt o;
     o.pen = pen != nullptr;
     helmholtz<double>(c, is_u, ds, S(c, 7), dr, cb, o, dt, n_sweeps, false, nullptr);
-    down_lone(c, sol, ds, kind);
+    down(c, sol, ds, kind);
     sync(c);
   });
 }
@@ -3018,12 +3032,10 @@ int fugu_vof_advection_tvd(fugu_ctx* c, const double* c_in, double* c_out, const
     double* dv = upk(c, 2, v, K_V);
     const bool fl = flux_x && flux_y;
     vof(c, ci, S(c, 3), du, dv, dt, fl ? S(c, 4) : nullptr, fl ? S(c, 5) : nullptr);
+    down(c, c_out, S(c, 3), K_CELL);
     if (fl) {
-      down(c, c_out, S(c, 3), K_CELL);
       down(c, flux_x, S(c, 4), K_U);
       down(c, flux_y, S(c, 5), K_V);
-    } else {
-      down_lone(c, c_out, S(c, 3), K_CELL);
     }
     sync(c);
   });
@@ -3038,7 +3050,7 @@ int fugu_svof_helmholtz_filter(fugu_ctx* c, const double* c_raw, double* c_smoot
     fugu_stats st{};
     collect(c, &st);
     if (iters_out) *iters_out = st.svof_iters;
-    down_lone(c, c_smooth, S(c, 1), K_CELL);
+    down(c, c_smooth, S(c, 1), K_CELL);
     sync(c);
   });
 }
@@ -3047,7 +3059,7 @@ int fugu_compute_interface_curvature(fugu_ctx* c, const double* c_smooth, double
   return guard(c, [&] {
     double* cs = upk(c, 0, c_smooth, K_CELL);
     curvature(c, cs, S(c, 1));
-    down_lone(c, kappa_curv, S(c, 1), K_CELL);
+    down(c, kappa_curv, S(c, 1), K_CELL);
     sync(c);
   });
 }
